@@ -5,6 +5,7 @@
 
 #include <cuda_runtime.h>
 #include <atomic>
+#include <cmath>
 #include <cstdint>
 #include <cstdio>
 #include <string>
@@ -34,6 +35,26 @@ __host__ __device__ inline cplx ccmul(cplx a, cplx b) {
   return make_double2(a.x * b.x + a.y * b.y, a.x * b.y - a.y * b.x);
 }
 __host__ __device__ inline double cabs2(cplx a) { return a.x * a.x + a.y * a.y; }
+
+// sqrt(a^2 + b^2 + c^2) with the largest magnitude factored out (dlapy3).
+__device__ __forceinline__ double hypot3(double a, double b, double c) {
+  a = fabs(a); b = fabs(b); c = fabs(c);
+  const double w = fmax(a, fmax(b, c));
+  if (w == 0.0) return 0.0;
+  a /= w; b /= w; c /= w;
+  return w * sqrt(a * a + b * b + c * c);
+}
+
+// 1 / z by Smith's algorithm (R. L. Smith, "Algorithm 116: Complex
+// division", CACM 5(8), 1962), which never squares |z|.
+__device__ __forceinline__ cplx recip_smith(cplx z) {
+  if (fabs(z.x) >= fabs(z.y)) {
+    const double r = z.y / z.x, t = 1.0 / (z.x + z.y * r);
+    return make_double2(t, -r * t);
+  }
+  const double r = z.x / z.y, t = 1.0 / (z.y + z.x * r);
+  return make_double2(r * t, -t);
+}
 
 // Error carrying a status code; every C-ABI function catches it.
 struct Error : public std::runtime_error {

@@ -259,19 +259,20 @@ static int site_factor(Context& c, MpsDev& s, int pos, char dir, cplx* r00, int 
     v.rd = 1; v.r0 = 0; v.r1 = Dl; v.cd = 1; v.c0 = 0; v.c1 = 1; v.conj = true;
   }
   int K = std::min(m, n);
-  dbuf_reserve(c, c.matA, (long long)m * n);
-  dbuf_reserve(c, c.matQ, (long long)m * K);
   dbuf_reserve(c, c.matR, (long long)K * n);
-  gather2(c.st(), m, n, s.A[pos].p, v, c.matA.p);
+  const bool direct = cutD <= 0 && cluster_qr_fits(m, n);  // reads and writes the site through the views
+  if (!direct) {
+    dbuf_reserve(c, c.matA, (long long)m * n);
+    dbuf_reserve(c, c.matQ, (long long)m * K);
+    gather2(c.st(), m, n, s.A[pos].p, v, c.matA.p);
+  }
   if (cutD > 0) {
     std::vector<double> sv;
     K = svd_cut(c.st(), m, n, c.matA.p, m, cutD, c.matQ.p, c.matR.p, sv, c.scratch);
     if (disc)
       for (size_t j = K; j < sv.size(); j++) *disc += sv[j] * sv[j];
-  } else {
-    householder_qr_inplace(c.st(), m, n, c.matA.p, c.matQ.p, m, c.matR.p, K, c.qrws);
   }
-  // write the isometry back into the site
+  // the isometry goes back into the site
   View2 w;
   if (dir == 'R') {
     s.dims[pos] = {d, Dl, K};
@@ -281,7 +282,12 @@ static int site_factor(Context& c, MpsDev& s, int pos, char dir, cplx* r00, int 
     // site X'(k, s, r) at k + K (s + d r) = conj(Q'(c = s + d r, k))
     w.rd = 1; w.r0 = 0; w.r1 = K; w.cd = 1; w.c0 = 0; w.c1 = 1; w.conj = true;
   }
-  scatter2(c.st(), m, K, c.matQ.p, s.A[pos].p, w);
+  if (direct) {
+    cluster_qr(c.st(), m, n, s.A[pos].p, v, s.A[pos].p, w, c.matR.p, K, c.qrws);
+  } else {
+    if (cutD <= 0) householder_qr_inplace(c.st(), m, n, c.matA.p, c.matQ.p, m, c.matR.p, K, c.qrws);
+    scatter2(c.st(), m, K, c.matQ.p, s.A[pos].p, w);
+  }
   if (r00 && K == 1 && n == 1) {
     MPSGPU_CUDA(cudaMemcpyAsync(r00, c.matR.p, sizeof(cplx), cudaMemcpyDeviceToHost, c.stream));
     MPSGPU_CUDA(cudaStreamSynchronize(c.stream));

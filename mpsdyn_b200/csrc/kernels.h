@@ -355,6 +355,11 @@ int svd_cut(const Stream& st, int m, int n, const cplx* A, long long lda, int cu
             std::vector<double>& sv, Scratch& scratch, bool left_s = false);
 
 // ---- Householder QR (LAPACK zgeqrf/zungqr conventions) ----
+// Complex flops (8 per complex MAC) of the factorisation and the explicit Q.
+inline double qr_flops(double m, double n) {
+  const double K = m < n ? m : n;
+  return 16.0 * (2.0 * m * n * K - (m + n) * K * K + 2.0 * K * K * K / 3.0);
+}
 // Factor the m x n column-major matrix A (ld = m; overwritten by R above and
 // the reflectors below the diagonal).  Q (m x K, ld = ldq) and R (K x n,
 // ld = ldr, zero below the diagonal) are written when non-null; K = min(m, n).
@@ -370,6 +375,12 @@ struct View2 {
   long long rd = 1, r0 = 1, r1 = 0, cd = 1, c0 = 0, c1 = 0;
   bool conj = false;
 };
+// The same factorisation in one thread-block cluster (qr_cluster.cu), A read
+// and Q written through strided views; A is not modified and may be Q's
+// buffer.  For matrices that cluster_qr_fits.
+bool cluster_qr_fits(int m, int n);
+void cluster_qr(const Stream& st, int m, int n, const cplx* A, const View2& va, cplx* Q, const View2& vq, cplx* R,
+                long long ldr, Scratch& scratch);
 // dst (m x n, col-major, ld m) = view(src)
 void gather2(const Stream& st, int m, int n, const cplx* src, const View2& v, cplx* dst);
 // view(dst) = src (m x n, col-major, ld m)
