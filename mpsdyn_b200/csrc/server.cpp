@@ -327,9 +327,17 @@ mpsgpu_status mpsgpu_server_cancel(mpsgpu_server* s, uint64_t id) {
     }
   }
   auto a = s->active.find(id);
-  if (a == s->active.end()) return MPSGPU_INVALID;
-  raise_cancel(*a->second);
-  return MPSGPU_OK;
+  if (a != s->active.end()) {
+    raise_cancel(*a->second);
+    return MPSGPU_OK;
+  }
+  for (auto& res : s->done) {  // finished, its result not collected yet
+    if (res.id == id) {
+      res.status = MPSGPU_CANCELLED;
+      return MPSGPU_OK;
+    }
+  }
+  return MPSGPU_INVALID;
 }
 
 mpsgpu_status mpsgpu_server_drain(mpsgpu_server* s, double timeout_s) {
