@@ -1087,9 +1087,12 @@ cplx contract2(Context& c, const MpoDev& ops, const MpsDev& ket, const MpsDev& b
 // for a batch of independent local problems advanced in lockstep.
 // Thick-restarted Lanczos with full reorthogonalisation, FP64; convergence
 // ||r|| <= tol * max|Ritz|.  Every task's product computes y = (H - sigma) x
-// (the excited-state multiplier without its projector); sigma follows the
-// task's latest Ritz value (shift0 before the first one is known), which
-// keeps the Gram-Schmidt passes well conditioned.  With nu > 0, U (N x nu)
+// (the excited-state multiplier without its projector).  sigma is the latest
+// diagonal element (shift0, near the lowest eigenvalue, for the first
+// product, and the sweep's last one until the first of a solve is known), so
+// that y has only a small component along v_j: with sigma at the lowest Ritz
+// value that component was about twice the rest of y, and nearly every step
+// failed the Gram-Schmidt test and took its second pass.  With nu > 0, U (N x nu)
 // holds the projector vectors with the square roots of the penalties folded
 // in, and the step adds U (U^H v_j) to every product
 // (TensorMultiplierProjMulti.cpp:81-90).
@@ -1227,7 +1230,8 @@ struct LzState {
   bool pending_restart = false;  // next round starts a new cycle at j0
   std::vector<double> a, b, s, gq;
   std::vector<cplx> gqc;
-  double theta = 0.0, step_hint = 0.0, sigma = 0.0;
+  double theta = 0.0, step_hint = 0.0;
+  double sigma0 = 0.0, sigma = 0.0;  // shift of the products: of iteration 0, of the next ones
   bool have_theta = false;
   TridiagLowest tri;
   ThickRestart thick;
@@ -1242,7 +1246,6 @@ void lanczos_batch(Context& c, std::vector<LzTask*>& tasks) {
   const int nt = (int)tasks.size();
   if (nt == 0) return;
   std::vector<LzState> S(nt);
-  long long nrb_total = 0;
   double* d_tmp = c.dscal + 512;
   for (int q = 0; q < nt; q++) {
     LzTask& t = *tasks[q];
@@ -1257,10 +1260,10 @@ void lanczos_batch(Context& c, std::vector<LzTask*>& tasks) {
     z.keep = std::max(1, z.m / 2);
     // budget of about 3840 products (60 cycles of a 64-vector space), whatever m
     z.max_restarts = std::max(60, 3840 / std::max(1, z.m - z.keep));
-    z.sigma = std::isfinite(t.shift0) ? t.shift0 : 0.0;
+    z.sigma0 = std::isfinite(t.shift0) ? t.shift0 : 0.0;
+    z.sigma = t.mid && std::isfinite(*t.mid) ? *t.mid : z.sigma0;
     dbuf_reserve(c, ws.V, (long long)N * (z.m + 1));
     dbuf_reserve(c, ws.w, N);
-    nrb_total += ceil_div(N, lanczos_step_rows_per_block());
     // v0 = x / ||x|| (a zero or non-finite start becomes the flat vector)
     dznrm2(st, N, t.x, d_tmp, c.scratch);
     MPSGPU_CUDA(cudaMemcpyAsync(c.hscal, d_tmp, sizeof(double), cudaMemcpyDeviceToHost, c.stream));
@@ -1272,18 +1275,12 @@ void lanczos_batch(Context& c, std::vector<LzTask*>& tasks) {
     zscal_inv(st, N, t.x, d_tmp, ws.V.p);
     t.iters = 0;
   }
-  // workspace of the step, shared by the instances of a launch: partial dots
-  // (row blocks x 256), two partial-norm arrays, the coefficients h, h2
-  dbuf_reserve(c, c.lzws, 2 * nrb_total * 256 + nrb_total + 8);
-  cplx* part = c.lzws.p;
-  cplx* part2 = part + nrb_total * 256;
-  double* pn1 = reinterpret_cast<double*>(part2 + nrb_total * 256);
-  double* pn2 = pn1 + nrb_total;
+  dbuf_reserve(c, c.lzws, lanczos_step_workspace(device_sms(c)));
 
   auto check_step = [&]() {
     if (*c.hlz_err) {
       MPSGPU_CUDA(cudaStreamSynchronize(c.stream));
-      MPSGPU_CUDA(cudaMemsetAsync(c.dcounter + kLzBarrierOffset, 0, 2 * LZ_MAXI * sizeof(unsigned), c.stream));
+      MPSGPU_CUDA(cudaMemsetAsync(c.dcounter, 0, kCounterWords * sizeof(unsigned), c.stream));
       MPSGPU_CUDA(cudaStreamSynchronize(c.stream));
       *c.hlz_err = 0;
       throw Error(MPSGPU_TIMEOUT, "lanczos: a bounded grid barrier of the Lanczos step ran out");
@@ -1304,18 +1301,14 @@ void lanczos_batch(Context& c, std::vector<LzTask*>& tasks) {
       LzState& z = S[it.first];
       LzTask& t = *z.t;
       if (rb.g1.n + 2 > GEMM_MAXP || rb.g3.n + 1 > GEMM_MAXP) flush();
-      t.product(c, t.ws->V.p + (long long)it.second * t.N, t.ws->w.p, z.sigma, rb);
+      const double sigma = it.second == 0 ? z.sigma0 : z.sigma;
+      t.product(c, t.ws->V.p + (long long)it.second * t.N, t.ws->w.p, sigma, rb);
     }
     flush();
     split_round_run(c, rb.sr);
     for (size_t i0 = 0; i0 < items.size(); i0 += LZ_MAXI) {
       LzBatch b;
       b.ninst = (int)std::min<size_t>(LZ_MAXI, items.size() - i0);
-      b.part = part;
-      b.part2 = part2;
-      b.pn1 = pn1;
-      b.pn2 = pn2;
-      b.bar = c.dcounter + kLzBarrierOffset;
       b.err = c.dlz_err;
       for (int i = 0; i < b.ninst; i++) {
         LzState& z = S[items[i0 + i].first];
@@ -1328,14 +1321,14 @@ void lanczos_batch(Context& c, std::vector<LzTask*>& tasks) {
         in.nu = t.nu;
         in.U = t.U;
         in.write_next = j + 1 < z.m ? 1 : 0;
-        in.sigma = z.sigma;
+        in.sigma = j == 0 ? z.sigma0 : z.sigma;
         in.V = t.ws->V.p;
         in.ldv = t.N;
         in.w = t.ws->w.p;
         in.sc = t.ws->dsc;
         in.mirror = t.ws->hsc_dev;
       }
-      lanczos_step(st, b);
+      lanczos_step(st, b, c.lzws.p, c.dcounter, c.lz_parity);
     }
     MPSGPU_CUDA(cudaEventRecord(ev, c.stream));
     for (auto& it : items) {
@@ -1402,7 +1395,6 @@ void lanczos_batch(Context& c, std::vector<LzTask*>& tasks) {
     // the coupling of V[:, r-1] to the new V[:, r], used by the next step
     MPSGPU_CUDA(cudaMemcpyAsync(&t.ws->dsc->beta[r - 1], &z.b[r - 1], sizeof(double), cudaMemcpyHostToDevice,
                                 c.stream));
-    z.sigma = z.theta;
     z.j0 = r;
     return false;
   };
@@ -1458,7 +1450,12 @@ void lanczos_batch(Context& c, std::vector<LzTask*>& tasks) {
         z.tri.solve(z.a, z.b, (int)z.a.size(), z.theta, z.s, normT);
       z.step_hint = z.have_theta ? std::fabs(th_old - z.theta) : 0.0;
       z.have_theta = true;
-      z.sigma = z.theta;
+      // the diagonal elements settle in the middle of the spectrum after the
+      // first one (the start vector is near the lowest eigenvector)
+      if (j > 0) {
+        z.sigma = alpha;
+        if (t.mid) *t.mid = alpha;
+      }
       const double res = beta * std::fabs(z.s[j]);
       const double scale = std::max(normT, std::fabs(z.theta));
       if (res <= t.tol * scale || beta <= 1e-14 * scale || j + 1 == t.N) {
@@ -1740,6 +1737,7 @@ struct GsSweep {
   LzWork& ws;
   int D = 0, L = 0;
   double offset = 0.0, tol = 1e-12;
+  double mid = std::nan("");  // middle of the local spectrum (LzTask::mid)
   EnvCache E;
   double energy = 0.0, val = 0.0;
   bool right = true, done = false;
@@ -1785,6 +1783,7 @@ struct GsSweep {
     t.x = init.A[pos].p;
     t.tol = split_phase ? std::max(tol, kSplitEigTol) : first64 ? std::max(tol, kFirst64EigTol) : tol;
     t.shift0 = val + offset;
+    t.mid = &mid;
     t.max_krylov = opt.max_krylov;
     t.ws = &ws;
     t.cnt = &cnt;
@@ -2193,6 +2192,7 @@ struct ExcSweep {
   std::vector<const MpsDev*> levels;
   int D = 0, L = 0, nk = 0;
   double offset = 0.0, tol = 1e-12;
+  double mid = std::nan("");  // middle of the local spectrum (LzTask::mid)
   EnvCache E;
   std::vector<EnvCache> NC;
   DBuf Lh, Rth, U;
@@ -2303,6 +2303,7 @@ struct ExcSweep {
     t.x = init.A[pos].p;
     t.tol = split_phase ? std::max(tol, kSplitEigTol) : first64 ? std::max(tol, kFirst64EigTol) : tol;
     t.shift0 = val + offset;
+    t.mid = &mid;
     t.max_krylov = opt.max_krylov;
     t.U = U.p;
     t.nu = nk;

@@ -21,10 +21,8 @@ struct DBuf {
   long long cap = 0;  // complex elements
 };
 
-// Device words of a context (zero at rest): one barrier pair per instance of
-// a Lanczos-step launch, from kLzBarrierOffset.
-constexpr int kLzBarrierOffset = 0;
-constexpr int kCounterWords = 2 * LZ_MAXI;
+// Device words of a context: two sets of the Lanczos step's barrier words.
+constexpr int kCounterWords = 2 * LZ_MAXI * LZ_BAR_WORDS;
 // Descriptor ring of a context: slots of kDescSlotBytes.
 constexpr int kDescSlots = 8;
 constexpr size_t kDescSlotBytes = 64 * 1024;
@@ -95,7 +93,8 @@ struct Context {
   cplx* dcplx = nullptr;       // device complex scalars (dots)
   double* hscal = nullptr;     // pinned host mirror
   cplx* hcplx = nullptr;
-  unsigned* dcounter = nullptr;   // kCounterWords device words: the Lanczos step's barrier pairs
+  unsigned* dcounter = nullptr;   // kCounterWords device words: the Lanczos step's barriers
+  int lz_parity = 0;              // the set its next launch uses
   std::vector<cudaEvent_t> iter_ev;  // one per Lanczos iteration in flight
   cudaEvent_t ev = nullptr;
   cudaEvent_t mv0 = nullptr, mv1 = nullptr;
@@ -259,6 +258,7 @@ struct LzTask {
   int N = 0;
   cplx* x = nullptr;  // start vector in, normalised eigenvector out
   double tol = 1e-12, shift0 = 0.0;
+  double* mid = nullptr;  // a sweep's last diagonal element (NaN: none yet), the shift of the first products
   const cplx* U = nullptr;  // projector vectors (N x nu), sqrt(penalty) folded in
   int nu = 0;
   int max_krylov = 64;

@@ -286,15 +286,17 @@ struct LanczosScalars {
 // entry; on exit sc->alpha[j], sc->beta[j] (and the mirror) are set and, when
 // write_next, V[:, j+1] = w / beta_j.  With nu > 0, U (n x nu, ld n) holds the
 // projector vectors (sqrt of the penalty folded in) and w += U (U^H v_j)
-// first.  Workspaces: part and part2 nrb_total x 256 complex, pn1/pn2
-// nrb_total; bar 2 x LZ_MAXI unsigned words that are zero at rest (one pair
-// per instance).
+// first.  ws: lanczos_step_workspace complex entries, shared by the launches of
+// a stream; bars: 2 x LZ_MAXI x LZ_BAR_WORDS words, zero at first (two sets
+// that the launches of a stream use in turn, parity saying which is next: a
+// launch clears the other set for its successor).
 constexpr int LZ_THREADS = 256;
 constexpr int LZ_MAXI = 16;  // instances per launch
 constexpr int LZ_MAXU = 8;   // projector vectors per instance
+constexpr int LZ_BAR_WORDS = 4;  // barriers of a step
 struct LzInst {
   int n = 0, j = 0, k = 0, nu = 0, write_next = 0;
-  int rb0 = 0, nrb = 0;     // row blocks, filled by lanczos_step
+  int rows = 0;             // rows of a CTA, filled by lanczos_step
   int cta0 = 0, ncta = 0;   // the instance's CTAs, filled by lanczos_step
   double sigma = 0.0;
   cplx* V = nullptr;
@@ -305,18 +307,19 @@ struct LzInst {
   LanczosScalars* mirror = nullptr;
 };
 struct LzBatch {
-  int ninst = 0, nrb_total = 0;
+  int ninst = 0;
   LzInst in[LZ_MAXI];
+  // filled by lanczos_step
   cplx* part = nullptr;
   cplx* part2 = nullptr;
   double* pn1 = nullptr;
   double* pn2 = nullptr;
   unsigned* bar = nullptr;
+  unsigned* bar_next = nullptr;
   int* err = nullptr;  // set when a bounded barrier ran out
 };
-// Rows per row block (the unit of the workspaces' nrb counts).
-int lanczos_step_rows_per_block();
-void lanczos_step(const Stream& st, LzBatch& b);
+long long lanczos_step_workspace(int sms);
+void lanczos_step(const Stream& st, LzBatch& b, cplx* ws, unsigned* bars, int& parity);
 
 // out[0] = ||x||_2 (deterministic two-stage reduction)
 void dznrm2(const Stream& st, int n, const cplx* x, double* out, Scratch& scratch);
