@@ -1,0 +1,77 @@
+"""Edges of the block Jacobi SVD (one CTA up to 16 columns, pairs of blocks of 8
+on a cluster, on the grid above 256 columns, the global-memory form for long
+columns) against LAPACK: Schmidt values and SVD cuts of chains whose central
+bonds have the size in question.  Jacobi values carry a few ulps per sweep of
+the largest one: 1e-12.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def chain(L, d, D, seed):
+    rng = np.random.default_rng(seed)
+    bond = [int(min(D, d ** min(k, L - k))) for k in range(L + 1)]
+    return [(rng.standard_normal((d, a, r)) + 1j * rng.standard_normal((d, a, r))) / np.sqrt(2.0 * d * a)
+            for a, r in zip(bond, bond[1:])]
+
+
+def cut_left(sites, D):
+    """SVD cuts to D from the right end, the factor passed to the left."""
+    out, carry, dropped = [], np.eye(1), 0.0
+    for A in reversed(sites):
+        A = np.einsum("sar,rq->saq", A, carry)
+        d, a, q = A.shape
+        U, s, Vh = np.linalg.svd(A.transpose(1, 0, 2).reshape(a, d * q), full_matrices=False)
+        k = min(D, len(s))
+        dropped += np.sum(s[k:] ** 2)
+        out.append(Vh[:k].reshape(k, d, q).transpose(1, 0, 2))
+        carry = U[:, :k] * s[:k]
+    return out[::-1], carry[0, 0], dropped, s
+
+
+def overlap(x, y):
+    e = np.ones((1, 1))
+    for a, b in zip(x, y):
+        e = np.einsum("ab,sac,sbd->cd", e, a.conj(), b, optimize=True)
+    return e[0, 0]
+
+
+def schmidt(sites, pos):
+    left, _, _, _ = cut_left(sites, 1 << 30)  # right-canonical, then the left part's factor
+    R = np.eye(1)
+    for A in left[:pos]:
+        A = np.einsum("ab,sbr->sar", R, A)
+        R = np.linalg.qr(A.reshape(-1, A.shape[2]))[1]
+    s = np.linalg.svd(R, compute_uv=False) ** 2
+    return s / s.sum()
+
+
+@pytest.mark.parametrize("d,L,D", [(2, 2, 2), (2, 8, 15), (2, 9, 16), (2, 10, 17), (2, 12, 31), (2, 12, 33), (2, 12, 64),
+                                   (2, 14, 100), (3, 10, 129), (2, 16, 256), (2, 18, 257), (3, 12, 300)])
+def test_schmidt_values_match_lapack(ctx, d, L, D):
+    sites = chain(L, d, D, D)
+    psi = ctx.mps(sites)
+    got = np.sort(ctx.schmidt_values(psi, L // 2))[::-1]
+    psi.free()
+    want = np.sort(schmidt(sites, L // 2))[::-1]
+    n = min(len(got), len(want))
+    assert np.abs(got[:n] - want[:n]).max() < 1e-12 * want[0]
+    assert np.all(got[n:] < 1e-24)
+
+
+@pytest.mark.parametrize("d,L,D,cut", [(2, 6, 8, 3), (2, 9, 16, 7), (2, 10, 24, 20), (2, 12, 64, 16), (3, 8, 81, 40),
+                                       (2, 16, 200, 100), (2, 18, 280, 64), (3, 12, 300, 90)])
+def test_cuts_match_lapack(ctx, d, L, D, cut):
+    sites = chain(L, d, D, D + cut)
+    psi = ctx.mps(sites)
+    phi, discarded = psi.approximate(cut)
+    got, norm = phi.download()
+    psi.free()
+    phi.free()
+    want, wnorm, dropped, _ = cut_left(sites, cut)
+    assert abs(norm / abs(wnorm) - 1) < 1e-12
+    assert abs(discarded - dropped) < 1e-12 * max(dropped, abs(wnorm) ** 2)
+    assert abs(abs(overlap(got, want)) - 1) < 1e-11
+    assert abs(overlap(got, got) - 1) < 1e-11
