@@ -21,8 +21,21 @@
 // launch; tiles of all problems are numbered consecutively.  Operands are
 // streamed through a three-stage shared-memory ring filled by cp.async
 // (16-byte copies, zero-fill beyond the edges); complex entries stay
-// interleaved in shared memory and each product is four real DMMAs in
-// independent accumulators (re.re, -im.im, re.im, im.re).
+// interleaved in shared memory and each product is four real DMMAs, two into
+// each accumulator (re, im): at two registers a value that leaves room for
+// three CTAs per SM (with four accumulators two fit).  Groups of single-tile
+// problems (bonds up to 16) keep four independent accumulators (re.re, -im.im,
+// re.im, im.re): they are bound by the latency of one tile, and the chain of
+// dependent DMMAs (27 cycles each) is half as long.
+//
+// Bound by the FP64 tensor pipe (a DMMA per 4 cycles and SM) once a group has
+// tiles for every SM, by latency below.  Around the main loop, the epilogue of
+// heff_gemm1w took three times its instructions while it divided by the leg
+// dimensions for every term; it now walks the legs with the leg matrix staged
+// in the ring's space.  Measured: four Hermitian products (eight problems) at
+// D = 96, w = 5 in 30.6 us for the first contraction and 33.3 us for the last one
+// (38.4 us with clusters of 8), one product at D = 64, w = 3 in 9.0 and 10.0 us
+// (9.8 and 10.7 us).
 #include <cooperative_groups.h>
 
 #include <mutex>
@@ -70,23 +83,25 @@ struct Ring {
 };
 
 template <int BM, int BN>
-constexpr size_t ring_bytes() {
+__host__ __device__ constexpr size_t ring_bytes() {
   return sizeof(Ring<BM, BN>) > (size_t)BM * (BN + PADC) * sizeof(cplx) ? sizeof(Ring<BM, BN>)
                                                                        : (size_t)BM * (BN + PADC) * sizeof(cplx);
 }
 
-// Accumulators of a warp tile: [MT][NT][set][half]
-template <int BM, int BN>
+// Accumulators of a warp tile: [MT][NT][set][half], sets re, im (NS = 2) or
+// re.re, -im.im, re.im, im.re (NS = 4)
+template <int BM, int BN, int NS>
 struct Acc {
   static constexpr int WM = BM / 2, WN = BN / 2, MT = WM / 8, NT = WN / 8;
-  double v[MT][NT][4][2];
+  double v[MT][NT][NS][2];
 };
 
 // Main loop over k in [kbeg, kend): loadA(ring, stage, k0) / loadB(...)
 // issue the cp.async copies of one BK slab.
-template <int BM, int BN, class LA, class LB>
-__device__ __forceinline__ void mainloop(Ring<BM, BN>& r, Acc<BM, BN>& acc, int kbeg, int kend, LA loadA, LB loadB) {
-  using AC = Acc<BM, BN>;
+template <int BM, int BN, int NS, class LA, class LB>
+__device__ __forceinline__ void mainloop(Ring<BM, BN>& r, Acc<BM, BN, NS>& acc, int kbeg, int kend, LA loadA,
+                                         LB loadB) {
+  using AC = Acc<BM, BN, NS>;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int wm0 = (warp & 1) * AC::WM, wn0 = ((warp >> 1) & 1) * AC::WN, kg = warp >> 2;
   const int fr = lane >> 2, fc = lane & 3;
@@ -95,7 +110,7 @@ __device__ __forceinline__ void mainloop(Ring<BM, BN>& r, Acc<BM, BN>& acc, int 
 #pragma unroll
     for (int j = 0; j < AC::NT; j++)
 #pragma unroll
-      for (int s = 0; s < 4; s++) acc.v[i][j][s][0] = acc.v[i][j][s][1] = 0.0;
+      for (int s = 0; s < NS; s++) acc.v[i][j][s][0] = acc.v[i][j][s][1] = 0.0;
   const int nslab = kend > kbeg ? (kend - kbeg + BK - 1) / BK : 0;
 #pragma unroll
   for (int s = 0; s < STAGES - 1; s++) {
@@ -136,10 +151,11 @@ __device__ __forceinline__ void mainloop(Ring<BM, BN>& r, Acc<BM, BN>& acc, int 
       for (int i = 0; i < AC::MT; i++)
 #pragma unroll
         for (int j = 0; j < AC::NT; j++) {
+          constexpr int II = NS == 4 ? 1 : 0, RI = NS / 2, IR = NS - 1;
           dmma(acc.v[i][j][0][0], acc.v[i][j][0][1], are[i], bre[j]);
-          dmma(acc.v[i][j][1][0], acc.v[i][j][1][1], naim[i], bim[j]);
-          dmma(acc.v[i][j][2][0], acc.v[i][j][2][1], are[i], bim[j]);
-          dmma(acc.v[i][j][3][0], acc.v[i][j][3][1], aim[i], bre[j]);
+          dmma(acc.v[i][j][RI][0], acc.v[i][j][RI][1], are[i], bim[j]);
+          dmma(acc.v[i][j][II][0], acc.v[i][j][II][1], naim[i], bim[j]);
+          dmma(acc.v[i][j][IR][0], acc.v[i][j][IR][1], aim[i], bre[j]);
         }
     }
   }
@@ -149,9 +165,9 @@ __device__ __forceinline__ void mainloop(Ring<BM, BN>& r, Acc<BM, BN>& acc, int 
 
 // Accumulators -> shared tile Cs[m][n] (ld BN + PADC): the warp groups'
 // partial sums added in group order.  Every thread of the block calls it.
-template <int BM, int BN>
-__device__ __forceinline__ void acc_to_smem(const Acc<BM, BN>& acc, cplx* Cs) {
-  using AC = Acc<BM, BN>;
+template <int BM, int BN, int NS>
+__device__ __forceinline__ void acc_to_smem(const Acc<BM, BN, NS>& acc, cplx* Cs) {
+  using AC = Acc<BM, BN, NS>;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int wm0 = (warp & 1) * AC::WM, wn0 = ((warp >> 1) & 1) * AC::WN, kg = warp >> 2;
   const int fr = lane >> 2, fc = lane & 3;
@@ -165,8 +181,11 @@ __device__ __forceinline__ void acc_to_smem(const Acc<BM, BN>& acc, cplx* Cs) {
 #pragma unroll
           for (int h = 0; h < 2; h++) {
             const int m = wm0 + i * 8 + fr, n = wn0 + j * 8 + 2 * fc + h;
-            const cplx v =
-                make_double2(acc.v[i][j][0][h] + acc.v[i][j][1][h], acc.v[i][j][2][h] + acc.v[i][j][3][h]);
+            cplx v;
+            if constexpr (NS == 4)
+              v = make_double2(acc.v[i][j][0][h] + acc.v[i][j][1][h], acc.v[i][j][2][h] + acc.v[i][j][3][h]);
+            else
+              v = make_double2(acc.v[i][j][0][h], acc.v[i][j][1][h]);
             cplx& c = Cs[m * (BN + PADC) + n];
             c = g == 0 ? v : cadd(c, v);
           }
@@ -186,8 +205,8 @@ __device__ __forceinline__ int problem_of(const D* d, int n, int t) {
 // ---------------------------------------------------------------------------
 // heff_gemm1w
 // ---------------------------------------------------------------------------
-template <int BM, int BN>
-__global__ void __launch_bounds__(nthreads<BM>()) heff_gemm1w_kernel(const __grid_constant__ Gemm1wBatch b) {
+template <int BM, int BN, int NS>
+__global__ void __launch_bounds__(nthreads<BM>(), BM <= 32 ? 3 : 2) heff_gemm1w_kernel(const __grid_constant__ Gemm1wBatch b) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int NT_ = nthreads<BM>();
   Ring<BM, BN>& ring = *reinterpret_cast<Ring<BM, BN>*>(smem_raw);
@@ -236,36 +255,53 @@ __global__ void __launch_bounds__(nthreads<BM>()) heff_gemm1w_kernel(const __gri
       cp_async16(&r.B[st][kk][nt], ok ? d.B + k + boff[u] : d.B, ok);
     }
   };
-  Acc<BM, BN> acc;
-  mainloop<BM, BN>(ring, acc, 0, d.K, loadA, loadB);
+  Acc<BM, BN, NS> acc;
+  mainloop<BM, BN, NS>(ring, acc, 0, d.K, loadA, loadB);
   cplx* Cs = reinterpret_cast<cplx*>(smem_raw);
-  acc_to_smem<BM, BN>(acc, Cs);
+  constexpr int LD = BN + PADC;
+  // the leg matrix behind the tile, where the ring leaves room for it
+  const int nout = d.n_o0 * d.n_o1, nw = d.n_i0 * d.n_i1 * nout;
+  const cplx* Wp = d.Wm;
+  if (nw <= (int)((ring_bytes<BM, BN>() - BM * LD * sizeof(cplx)) / sizeof(cplx))) {
+    cplx* Ws = Cs + BM * LD;
+    for (int e = tid; e < nw; e += NT_) Ws[e] = __ldg(&d.Wm[e]);
+    Wp = Ws;
+  }
+  acc_to_smem<BM, BN, NS>(acc, Cs);
   __syncthreads();
-  // per pixel (x, y): out[o0 + n_o0 o1] = sum_{i0, i1} Wm[o, i0 + n_i0 i1] C[(x, i0), (i1, y)]
-  const int nin = d.n_i0 * d.n_i1, nout = d.n_o0 * d.n_o1;
-  const int npix = TX * TY;
-  for (int p = tid; p < npix * nout; p += NT_) {
-    const int o = p / npix, pix = p % npix;
+  // per pixel (x, y): out[o0 + n_o0 o1] = sum_{i0, i1} Wm[o, i0 + n_i0 i1] C[(x, i0), (i1, y)];
+  // ng threads per pixel, each every ng-th output, two at a time
+  const int npix = TX * TY, ng = max(1, NT_ / npix);
+  for (int p = tid; p < npix * ng; p += NT_) {
+    const int pix = p % npix, g = p / npix;
     const int xl = pix % TX, yl = pix / TX;
     const int x = x0 + xl, y = y0 + yl;
     if (x >= d.X || y >= d.Y) continue;
-    cplx s = make_double2(0.0, 0.0);
-    const cplx* wrow = d.Wm + o;
-    for (int i = 0; i < nin; i++) {
-      const int i0 = i % d.n_i0, i1 = i / d.n_i0;
-      const cplx c = Cs[(xl + TX * i0) * (BN + PADC) + (i1 + d.n_i1 * yl)];
-      s = cadd(s, cmul(__ldg(&wrow[(long long)nout * i]), c));
+    const cplx* cp = Cs + xl * LD + d.n_i1 * yl;
+    cplx* op = d.out + x * d.ox + y * d.oy;
+    for (int o = g; o < nout; o += 2 * ng) {
+      const int o2 = o + ng < nout ? o + ng : o;
+      cplx s = make_double2(0.0, 0.0), s2 = s;
+      const cplx* w = Wp;
+      for (int i1 = 0; i1 < d.n_i1; i1++) {
+        const cplx* c0 = cp + i1;
+        for (int i0 = 0; i0 < d.n_i0; i0++, c0 += TX * LD, w += nout) {
+          const cplx c = *c0;
+          s = cadd(s, cmul(w[o], c));
+          s2 = cadd(s2, cmul(w[o2], c));
+        }
+      }
+      op[(o % d.n_o0) * d.so0 + (o / d.n_o0) * d.so1] = s;
+      if (o2 != o) op[(o2 % d.n_o0) * d.so0 + (o2 / d.n_o0) * d.so1] = s2;
     }
-    const int o0 = o % d.n_o0, o1 = o / d.n_o0;
-    d.out[x * d.ox + y * d.oy + o0 * d.so0 + o1 * d.so1] = s;
   }
 }
 
 // ---------------------------------------------------------------------------
 // heff_gemm3 (cluster split-K)
 // ---------------------------------------------------------------------------
-template <int BM, int BN, int CS>
-__global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(nthreads<BM>())
+template <int BM, int BN, int CS, int NS>
+__global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(nthreads<BM>(), BM <= 32 ? 3 : 2)
     heff_gemm3_kernel(const __grid_constant__ Gemm3Batch b) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int NT_ = nthreads<BM>();
@@ -280,32 +316,44 @@ __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(nthreads<BM>())
   const int chunk = ((Ktot + CS - 1) / CS + BK - 1) / BK * BK;
   const int kbeg = min(Ktot, rank * chunk), kend = min(Ktot, kbeg + chunk);
   const int tid = threadIdx.x;
+  // the (row, k) and (k, column) slots this thread copies are the same in every
+  // slab: their rows and columns are tested once (-1 = outside)
+  constexpr int AE = BM * BK / NT_, BE = BN * BK / NT_;
+  int am[AE], bn[BE];
+#pragma unroll
+  for (int u = 0; u < AE; u++) {
+    const int m = m0 + (tid + u * NT_) % BM;
+    am[u] = m < d.M ? m : -1;
+  }
+#pragma unroll
+  for (int u = 0; u < BE; u++) {
+    const int n = n0 + (tid + u * NT_) / BK;
+    bn[u] = n < d.N ? n : -1;
+  }
   auto loadA = [&](Ring<BM, BN>& r, int st, int k0) {
 #pragma unroll
-    for (int e = tid; e < BM * BK; e += NT_) {
-      const int mt = e % BM, kk = e / BM;
-      const int m = m0 + mt, k = k0 + kk;
-      const bool ok = m < d.M && k < kend;
+    for (int u = 0; u < AE; u++) {
+      const int e = tid + u * NT_, mt = e % BM, kk = e / BM, k = k0 + kk;
+      const bool ok = am[u] >= 0 && k < kend;
       const cplx* src = d.A1;
-      if (ok) src = k < d.K1 ? d.A1 + m + (long long)k * d.lda1 : d.A2 + m + (long long)(k - d.K1) * d.lda2;
+      if (ok) src = k < d.K1 ? d.A1 + am[u] + (long long)k * d.lda1 : d.A2 + am[u] + (long long)(k - d.K1) * d.lda2;
       cp_async16(&r.A[st][kk][mt], src, ok);
     }
   };
   auto loadB = [&](Ring<BM, BN>& r, int st, int k0) {
 #pragma unroll
-    for (int e = tid; e < BN * BK; e += NT_) {
-      const int kk = e % BK, nt = e / BK;
-      const int n = n0 + nt, k = k0 + kk;
-      const bool ok = n < d.N && k < kend;
+    for (int u = 0; u < BE; u++) {
+      const int e = tid + u * NT_, kk = e % BK, nt = e / BK, k = k0 + kk;
+      const bool ok = bn[u] >= 0 && k < kend;
       const cplx* src = d.B1;
-      if (ok) src = k < d.K1 ? d.B1 + k + (long long)n * d.ldb1 : d.B2 + (k - d.K1) + (long long)n * d.ldb2;
+      if (ok) src = k < d.K1 ? d.B1 + k + (long long)bn[u] * d.ldb1 : d.B2 + (k - d.K1) + (long long)bn[u] * d.ldb2;
       cp_async16(&r.B[st][kk][nt], src, ok);
     }
   };
-  Acc<BM, BN> acc;
-  mainloop<BM, BN>(ring, acc, kbeg, kend, loadA, loadB);
+  Acc<BM, BN, NS> acc;
+  mainloop<BM, BN, NS>(ring, acc, kbeg, kend, loadA, loadB);
   cplx* Cs = reinterpret_cast<cplx*>(smem_raw);
-  acc_to_smem<BM, BN>(acc, Cs);
+  acc_to_smem<BM, BN, NS>(acc, Cs);
   // rows [r0, r1) of the tile are finished by this rank: the sum over the
   // ranks' partial tiles in rank order, then the epilogue
   constexpr int RPR = BM / CS;
@@ -314,7 +362,7 @@ __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(nthreads<BM>())
     cg::cluster_group cl = cg::this_cluster();
     cl.sync();
     for (int e = tid; e < RPR * BN; e += NT_) {
-      const int mt = r0 + e / BN, nt = e % BN;
+      const int mt = r0 + e % RPR, nt = e / RPR;
       const int m = m0 + mt, n = n0 + nt;
       cplx s = make_double2(0.0, 0.0);
 #pragma unroll
@@ -354,16 +402,15 @@ std::mutex g_heff_mu;
 void heff_setup() {
   if (!device_needs_setup(g_heff_setup)) return;
   std::lock_guard<std::mutex> lk(g_heff_mu);
-  set_smem(heff_gemm1w_kernel<64, 32>, ring_bytes<64, 32>());
-  set_smem(heff_gemm1w_kernel<32, 32>, ring_bytes<32, 32>());
-  set_smem(heff_gemm3_kernel<64, 32, 1>, ring_bytes<64, 32>());
-  set_smem(heff_gemm3_kernel<64, 32, 2>, ring_bytes<64, 32>());
-  set_smem(heff_gemm3_kernel<64, 32, 4>, ring_bytes<64, 32>());
-  set_smem(heff_gemm3_kernel<64, 32, 8>, ring_bytes<64, 32>());
-  set_smem(heff_gemm3_kernel<32, 32, 1>, ring_bytes<32, 32>());
-  set_smem(heff_gemm3_kernel<32, 32, 2>, ring_bytes<32, 32>());
-  set_smem(heff_gemm3_kernel<32, 32, 4>, ring_bytes<32, 32>());
-  set_smem(heff_gemm3_kernel<32, 32, 8>, ring_bytes<32, 32>());
+  set_smem(heff_gemm1w_kernel<64, 32, 2>, ring_bytes<64, 32>());
+  set_smem(heff_gemm1w_kernel<32, 32, 2>, ring_bytes<32, 32>());
+  set_smem(heff_gemm1w_kernel<32, 32, 4>, ring_bytes<32, 32>());
+  set_smem(heff_gemm3_kernel<64, 32, 1, 2>, ring_bytes<64, 32>());
+  set_smem(heff_gemm3_kernel<32, 32, 1, 4>, ring_bytes<32, 32>());
+  set_smem(heff_gemm3_kernel<32, 32, 1, 2>, ring_bytes<32, 32>());
+  set_smem(heff_gemm3_kernel<32, 32, 2, 2>, ring_bytes<32, 32>());
+  set_smem(heff_gemm3_kernel<32, 32, 4, 2>, ring_bytes<32, 32>());
+  set_smem(heff_gemm3_kernel<32, 32, 8, 2>, ring_bytes<32, 32>());
   mark_device_done(g_heff_setup);
 }
 
@@ -390,8 +437,10 @@ void heff_gemm1w(const Stream& st, Gemm1wBatch& b) {
   // chains at D = 128 as well as for one chain; 64 only for groups that fill
   // the GPU many times over
   long long t64 = 0;
+  bool single = true;  // every problem one 16 x 16 tile of pixels at most
   for (int q = 0; q < b.n; q++) {
     const Gemm1wDesc& d = b.d[q];
+    single = single && d.X <= 16 && d.Y <= 16;
     MPSGPU_CHECK(d.n_i0 >= 1 && d.n_i0 <= 32 && d.n_i1 >= 1 && d.n_i1 <= 32 && d.X > 0 && d.Y > 0 && d.K > 0,
                  MPSGPU_BAD_SHAPE, "gemm1w: leg dimensions");
     t64 += (long long)ceil_div(d.X, 64 / d.n_i0) * ceil_div(d.Y, 32 / d.n_i1);
@@ -414,9 +463,11 @@ void heff_gemm1w(const Stream& st, Gemm1wBatch& b) {
   }
   ProfScope ps(st, GemmProfiler::GEMM64, work);
   if (bm == 64)
-    heff_gemm1w_kernel<64, 32><<<tiles, nthreads<64>(), ring_bytes<64, 32>(), st.s>>>(b);
+    heff_gemm1w_kernel<64, 32, 2><<<tiles, nthreads<64>(), ring_bytes<64, 32>(), st.s>>>(b);
+  else if (single)
+    heff_gemm1w_kernel<32, 32, 4><<<tiles, nthreads<32>(), ring_bytes<32, 32>(), st.s>>>(b);
   else
-    heff_gemm1w_kernel<32, 32><<<tiles, nthreads<32>(), ring_bytes<32, 32>(), st.s>>>(b);
+    heff_gemm1w_kernel<32, 32, 2><<<tiles, nthreads<32>(), ring_bytes<32, 32>(), st.s>>>(b);
   after_launch(st);
 }
 
@@ -428,21 +479,25 @@ void heff_gemm3(const Stream& st, Gemm3Batch& b) {
   // CTA per SM
   long long t64 = 0, t32 = 0;
   int kmax = 0;
+  bool single = true;  // every problem at most one tile of a D = 16 site
   for (int q = 0; q < b.n; q++) {
     const Gemm3Desc& d = b.d[q];
+    single = single && d.M <= 32 && d.N <= 16;
     MPSGPU_CHECK(d.M > 0 && d.N > 0 && d.K1 > 0 && d.K2 >= 0, MPSGPU_BAD_SHAPE, "gemm3: shape");
     t64 += (long long)ceil_div(d.M, 64) * ceil_div(d.N, 32);
     t32 += (long long)ceil_div(d.M, 32) * ceil_div(d.N, 32);
     kmax = std::max(kmax, d.K1 + d.K2);
   }
   // 64-row tiles (two CTAs per SM by shared memory) once they alone fill the
-  // GPU twice; otherwise 32-row tiles (four per SM), with the K range split
-  // over a cluster while that keeps within one wave and K chunks of at
-  // least four slabs
+  // GPU twice; otherwise 32-row tiles, with the K range split over a cluster
+  // while the CTAs keep within two per SM (three fit, but clusters of 4 and 8
+  // do not pack the SMs of a GPC to the last one: at 576 CTAs in clusters of 8
+  // a third wave took 38 us where 288 in clusters of 4 take 33 us) and K chunks
+  // of at least four slabs
   int bm = 64, cs = 1;
   if (t64 < 2LL * nsm) {
     bm = 32;
-    while (cs < 8 && t32 * cs * 2 <= 4LL * nsm && kmax / (cs * 2) >= 4 * BK) cs *= 2;
+    while (!single && cs < 8 && t32 * cs * 2 <= 2LL * nsm && kmax / (cs * 2) >= 4 * BK) cs *= 2;
   }
   int tiles = 0;
   for (int q = 0; q < b.n; q++) {
@@ -456,18 +511,20 @@ void heff_gemm3(const Stream& st, Gemm3Batch& b) {
   double work = 0.0;
   for (int q = 0; q < b.n; q++) work += 8.0 * (double)b.d[q].M * b.d[q].N * (b.d[q].K1 + b.d[q].K2);
   ProfScope ps(st, GemmProfiler::GEMM64, work);
-#define MPSGPU_G3(BMv, CSv)                                                                   \
-  heff_gemm3_kernel<BMv, 32, CSv><<<grid, nthreads<BMv>(), ring_bytes<BMv, 32>(), st.s>>>(b)
+#define MPSGPU_G3(BMv, CSv, NSv)                                                                   \
+  heff_gemm3_kernel<BMv, 32, CSv, NSv><<<grid, nthreads<BMv>(), ring_bytes<BMv, 32>(), st.s>>>(b)
   if (bm == 64) {
-    MPSGPU_G3(64, 1);
+    MPSGPU_G3(64, 1, 2);
+  } else if (single) {
+    MPSGPU_G3(32, 1, 4);
   } else if (cs == 1) {
-    MPSGPU_G3(32, 1);
+    MPSGPU_G3(32, 1, 2);
   } else if (cs == 2) {
-    MPSGPU_G3(32, 2);
+    MPSGPU_G3(32, 2, 2);
   } else if (cs == 4) {
-    MPSGPU_G3(32, 4);
+    MPSGPU_G3(32, 4, 2);
   } else {
-    MPSGPU_G3(32, 8);
+    MPSGPU_G3(32, 8, 2);
   }
 #undef MPSGPU_G3
   after_launch(st);
