@@ -179,19 +179,6 @@ __global__ void zaxpby_kernel(int n, cplx a, const cplx* __restrict__ x, cplx b,
     y[i] = cadd(cmul(a, x[i]), cmul(b, y[i]));
 }
 
-__global__ void combine_real_kernel(int n, int k, const cplx* __restrict__ V, long long ldv,
-                                    const double* __restrict__ s, cplx* __restrict__ y) {
-  __shared__ double ss[256];
-  for (int t = threadIdx.x; t < k; t += blockDim.x) ss[t] = s[t];
-  __syncthreads();
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x) {
-    cplx acc = make_double2(0.0, 0.0);
-    for (int j = 0; j < k; j++) acc = cadd(acc, cscale(V[i + j * ldv], ss[j]));
-    y[i] = acc;
-  }
-}
-
 __global__ void zcopy_kernel(long long n, const cplx* __restrict__ s, cplx* __restrict__ d) {
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x)
@@ -362,12 +349,6 @@ void zscal_inv(const Stream& st, int n, const cplx* x, const double* nrm, cplx* 
 
 void zaxpby(const Stream& st, int n, cplx a, const cplx* x, cplx b, cplx* y) {
   zaxpby_kernel<<<grid_for(n), TPB, 0, st.s>>>(n, a, x, b, y);
-  after_launch(st);
-}
-
-void combine_real(const Stream& st, int n, int k, const cplx* V, long long ldv, const double* s, cplx* y) {
-  MPSGPU_CHECK(k <= 256, MPSGPU_BAD_SHAPE, "combine_real: k > 256");
-  combine_real_kernel<<<grid_for(n), TPB, 0, st.s>>>(n, k, V, ldv, s, y);
   after_launch(st);
 }
 

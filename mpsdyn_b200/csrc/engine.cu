@@ -1202,7 +1202,6 @@ void LzWork::init(Context& c) {
   MPSGPU_CUDA(cudaMemsetAsync(dsc, 0, sizeof(LanczosScalars), c.stream));
   MPSGPU_CUDA(cudaHostAlloc((void**)&hsc, sizeof(LanczosScalars), cudaHostAllocMapped));
   MPSGPU_CUDA(cudaHostGetDevicePointer((void**)&hsc_dev, hsc, 0));
-  MPSGPU_CUDA(cudaMalloc((void**)&dS, 256 * sizeof(double)));
 }
 
 void LzWork::release(Context& c) {
@@ -1211,11 +1210,9 @@ void LzWork::release(Context& c) {
     cudaStreamSynchronize(c.stream);
     cudaFree(dsc);
     cudaFreeHost(hsc);
-    cudaFree(dS);
   }
   dsc = nullptr;
   hsc = hsc_dev = nullptr;
-  dS = nullptr;
 }
 
 namespace {
@@ -1246,7 +1243,6 @@ void lanczos_batch(Context& c, std::vector<LzTask*>& tasks) {
   const int nt = (int)tasks.size();
   if (nt == 0) return;
   std::vector<LzState> S(nt);
-  double* d_tmp = c.dscal + 512;
   for (int q = 0; q < nt; q++) {
     LzTask& t = *tasks[q];
     LzState& z = S[q];
@@ -1264,15 +1260,6 @@ void lanczos_batch(Context& c, std::vector<LzTask*>& tasks) {
     z.sigma = t.mid && std::isfinite(*t.mid) ? *t.mid : z.sigma0;
     dbuf_reserve(c, ws.V, (long long)N * (z.m + 1));
     dbuf_reserve(c, ws.w, N);
-    // v0 = x / ||x|| (a zero or non-finite start becomes the flat vector)
-    dznrm2(st, N, t.x, d_tmp, c.scratch);
-    MPSGPU_CUDA(cudaMemcpyAsync(c.hscal, d_tmp, sizeof(double), cudaMemcpyDeviceToHost, c.stream));
-    MPSGPU_CUDA(cudaStreamSynchronize(c.stream));
-    if (!(c.hscal[0] > 0.0) || !std::isfinite(c.hscal[0])) {
-      zfill(st, N, make_double2(1.0 / std::sqrt((double)N), 0.0), t.x);
-      dznrm2(st, N, t.x, d_tmp, c.scratch);
-    }
-    zscal_inv(st, N, t.x, d_tmp, ws.V.p);
     t.iters = 0;
   }
   dbuf_reserve(c, c.lzws, lanczos_step_workspace(device_sms(c)));
@@ -1340,14 +1327,35 @@ void lanczos_batch(Context& c, std::vector<LzTask*>& tasks) {
       if (S[it.first].t->cnt) S[it.first].t->cnt->host_launch_s += dt;
   };
 
-  // Ritz vector of a task's tridiagonal (k x k) into its x, normalised (enqueued)
-  auto ritz_vector = [&](LzState& z, int k) {
+  // Normalised combinations, grouped: the start vectors v0 = x / |x|, and the
+  // Ritz vectors of tasks' tridiagonals (k x k) into their x (enqueued)
+  LzCombineBatch cb;
+  int cb_s = 0;
+  auto combine_flush = [&]() {
+    if (cb.ninst == 0) return;
+    cb.err = c.dlz_err;
+    lanczos_combine(st, cb, c.lzws.p, c.dcounter, c.lz_parity);
+    cb.ninst = 0;
+    cb_s = 0;
+  };
+  auto combine_add = [&](LzState& z, int k) {
     LzTask& t = *z.t;
-    MPSGPU_CUDA(cudaMemcpyAsync(t.ws->dS, z.s.data(), k * sizeof(double), cudaMemcpyHostToDevice, c.stream));
-    combine_real(st, t.N, k, t.ws->V.p, t.N, t.ws->dS, t.x);
-    dznrm2(st, t.N, t.x, d_tmp, c.scratch);
-    zscal_inv(st, t.N, t.x, d_tmp, t.x);
-    t.theta = z.theta;
+    if (cb.ninst == LZ_MAXI || cb_s + k > LZ_COMBINE_S) combine_flush();
+    LzCombine& in = cb.in[cb.ninst++];
+    in.n = t.N;
+    in.k = k;
+    in.s0 = cb_s;
+    in.V = k > 0 ? t.ws->V.p : t.x;
+    in.ldv = t.N;
+    in.out = k > 0 ? t.x : t.ws->V.p;
+    std::copy(z.s.begin(), z.s.begin() + k, cb.s + cb_s);
+    cb_s += k;
+  };
+  for (auto& z : S) combine_add(z, 0);
+  combine_flush();
+  auto ritz_vector = [&](LzState& z, int k) {
+    combine_add(z, k);
+    z.t->theta = z.theta;
     z.done = true;
   };
 
@@ -1359,6 +1367,7 @@ void lanczos_batch(Context& c, std::vector<LzTask*>& tasks) {
     if (z.keep >= m) {
       // no room to keep more than one vector: restart from the Ritz vector
       ritz_vector(z, m);
+      combine_flush();
       z.done = false;
       zcopy(st, N, t.x, t.ws->V.p);
       z.a.clear();
@@ -1469,6 +1478,7 @@ void lanczos_batch(Context& c, std::vector<LzTask*>& tasks) {
       }
       if (t.cnt) t.cnt->host_tridiag_s += secs(t0, clk::now());
     }
+    combine_flush();
     cur = std::move(nxt);
     cur_ev = nxt_ev;
     // tasks that restarted (or stopped speculating) and are not in the round

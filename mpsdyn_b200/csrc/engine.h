@@ -42,7 +42,6 @@ struct LzWork {
   LanczosScalars* dsc = nullptr;
   LanczosScalars* hsc = nullptr;
   LanczosScalars* hsc_dev = nullptr;
-  double* dS = nullptr;
   void init(Context& c);
   void release(Context& c);
 };

@@ -320,6 +320,29 @@ struct LzBatch {
 };
 long long lanczos_step_workspace(int sms);
 void lanczos_step(const Stream& st, LzBatch& b, cplx* ws, unsigned* bars, int& parity);
+// Normalised combinations of a group in one launch: out = y / |y|, y = sum_l
+// s[s0 + l] V[:, l] (k > 0; s real), or y = V[:, 0] (k = 0: a start vector; a
+// zero or non-finite one becomes the flat vector).  ws, bars and parity as for
+// lanczos_step.
+struct LzCombine {
+  int n = 0, k = 0, s0 = 0;
+  int rows = 0, cta0 = 0, ncta = 0;  // filled by lanczos_combine
+  const cplx* V = nullptr;
+  long long ldv = 0;
+  cplx* out = nullptr;
+};
+constexpr int LZ_COMBINE_S = 1024;  // coefficients of a launch
+struct LzCombineBatch {
+  int ninst = 0;
+  LzCombine in[LZ_MAXI];
+  double s[LZ_COMBINE_S];
+  int* err = nullptr;
+  // filled by lanczos_combine
+  double* pn = nullptr;
+  unsigned* bar = nullptr;
+  unsigned* bar_next = nullptr;
+};
+void lanczos_combine(const Stream& st, LzCombineBatch& b, cplx* ws, unsigned* bars, int& parity);
 
 // out[0] = ||x||_2 (deterministic two-stage reduction)
 void dznrm2(const Stream& st, int n, const cplx* x, double* out, Scratch& scratch);
@@ -327,9 +350,6 @@ void dznrm2(const Stream& st, int n, const cplx* x, double* out, Scratch& scratc
 void zscal_inv(const Stream& st, int n, const cplx* x, const double* nrm, cplx* y);
 // y = a x + b y (host scalars)
 void zaxpby(const Stream& st, int n, cplx a, const cplx* x, cplx b, cplx* y);
-// y = sum_j s[j] V[:, j]  (s real, device)
-void combine_real(const Stream& st, int n, int k, const cplx* V, long long ldv, const double* s,
-                  cplx* y);
 // dst = src (n complex)
 void zcopy(const Stream& st, int n, const cplx* src, cplx* dst);
 void zfill(const Stream& st, long long n, cplx v, cplx* dst);

@@ -442,6 +442,46 @@ __global__ void __launch_bounds__(T, 2) lanczos_step_kernel(const __grid_constan
   }
 }
 
+// ---- normalised combinations: the start vector of a solve and its Ritz vector ----
+// out = y / |y| with y = sum_l s_l V[:, l] (k > 0) or y = V[:, 0] (k = 0), of a
+// group of instances in one cooperative launch: rows of y stay in shared memory
+// across the barrier that closes the norms.  k = 0 replaces a zero or
+// non-finite y by the flat vector.
+__global__ void __launch_bounds__(T, 2) lanczos_combine_kernel(const __grid_constant__ LzCombineBatch b) {
+  __shared__ cplx ysm[WCAP];
+  __shared__ double ss[KMAXS], redn[NW];
+  const int tid = threadIdx.x;
+  if (blockIdx.x == 0 && tid < LZ_MAXI * PHASES) b.bar_next[tid] = 0;
+  int q = 0;
+  while (q + 1 < b.ninst && b.in[q + 1].cta0 <= (int)blockIdx.x) q++;
+  const LzCombine& in = b.in[q];
+  const int rank = (int)blockIdx.x - in.cta0, k = in.k;
+  const int r0 = rank * in.rows, n = min(in.rows, in.n - r0);
+  cplx* y = n <= WCAP ? ysm : in.out + r0;
+  for (int l = tid; l < k; l += T) ss[l] = b.s[in.s0 + l];
+  __syncthreads();
+  double s2 = 0.0;
+  for (int r = tid; r < n; r += T) {
+    const cplx* v = in.V + r0 + r;
+    cplx a = make_double2(0.0, 0.0);
+    if (k == 0) a = v[0];
+#pragma unroll 8
+    for (int l = 0; l < k; l++) {
+      const cplx x = __ldcg(v + (long long)l * in.ldv);
+      a.x = fma(ss[l], x.x, a.x);
+      a.y = fma(ss[l], x.y, a.y);
+    }
+    y[r] = a;
+    s2 += cabs2(a);
+  }
+  block_sum_to(s2, redn, &b.pn[in.cta0 + rank]);
+  if (!group_barrier(b.bar + PHASES * q, in.ncta, b.err)) return;
+  const double nrm = sqrt(sum_norms(b.pn + in.cta0, in.ncta)), inv = 1.0 / nrm;
+  const bool flat = k == 0 && !(nrm > 0.0 && nrm < __longlong_as_double(0x7ff0000000000000ll));
+  const double f = 1.0 / sqrt((double)in.n);
+  for (int r = tid; r < n; r += T) in.out[r0 + r] = flat ? make_double2(f, 0.0) : cscale(y[r], inv);
+}
+
 std::atomic<unsigned long long> g_lz_setup{0};
 int g_lz_sms[64] = {0};
 
@@ -451,6 +491,51 @@ int g_lz_sms[64] = {0};
 // of partial norms for at most two CTAs per SM.
 static int lz_max_ctas(int sms) { return 2 * sms; }
 long long lanczos_step_workspace(int sms) { return 2LL * lz_max_ctas(sms) * KMAXS + lz_max_ctas(sms); }
+
+// One-time set-up of the device's kernels; its SM count.
+static int lz_setup() {
+  int dev = 0;
+  MPSGPU_CUDA(cudaGetDevice(&dev));
+  MPSGPU_CHECK(dev < 64, MPSGPU_INVALID, "lanczos step: device number");
+  if (device_needs_setup(g_lz_setup)) {
+    int nsm = 148;
+    MPSGPU_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    for (const void* f : {(const void*)lanczos_step_kernel<false>, (const void*)lanczos_step_kernel<true>,
+                          (const void*)lanczos_combine_kernel}) {
+      int per = 0;
+      MPSGPU_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, f, T, 0));
+      MPSGPU_CHECK(per >= 2, MPSGPU_BAD_SHAPE, "lanczos step: kernel does not fit twice on an SM");
+    }
+    g_lz_sms[dev] = nsm;
+    mark_device_done(g_lz_setup);
+  }
+  return g_lz_sms[dev];
+}
+
+void lanczos_combine(const Stream& st, LzCombineBatch& b, cplx* ws, unsigned* bars, int& parity) {
+  MPSGPU_CHECK(b.ninst >= 1 && b.ninst <= LZ_MAXI, MPSGPU_BAD_SHAPE, "lanczos combine: group size");
+  const int G = lz_max_ctas(lz_setup());
+  long long rows = 0;
+  for (int q = 0; q < b.ninst; q++) rows += b.in[q].n;
+  // a row per thread until every slot has a CTA
+  const int per = std::max(T, ceil_div(ceil_div(rows, G - b.ninst), 32) * 32);
+  int c0 = 0;
+  for (int q = 0; q < b.ninst; q++) {
+    LzCombine& in = b.in[q];
+    MPSGPU_CHECK(in.n > 0 && in.k >= 0 && in.k <= KMAXS, MPSGPU_BAD_SHAPE, "lanczos combine: sizes");
+    in.rows = per;
+    in.ncta = ceil_div(in.n, per);
+    in.cta0 = c0;
+    c0 += in.ncta;
+  }
+  b.pn = reinterpret_cast<double*>(ws);
+  b.bar = bars + parity * LZ_MAXI * PHASES;
+  parity ^= 1;
+  b.bar_next = bars + parity * LZ_MAXI * PHASES;
+  void* args[] = {&b};
+  MPSGPU_CUDA(cudaLaunchCooperativeKernel((void*)lanczos_combine_kernel, dim3(c0), dim3(T), args, 0, st.s));
+  after_launch(st);
+}
 
 void lanczos_step(const Stream& st, LzBatch& b, cplx* ws, unsigned* bars, int& parity) {
   MPSGPU_CHECK(b.ninst >= 1 && b.ninst <= LZ_MAXI, MPSGPU_BAD_SHAPE, "lanczos step: group size");
@@ -465,18 +550,7 @@ void lanczos_step(const Stream& st, LzBatch& b, cplx* ws, unsigned* bars, int& p
     kmax = std::max(kmax, in.k);
     wsum += (double)in.n * (2.0 * in.k + 6.0 + 2.0 * in.nu);
   }
-  int dev = 0;
-  MPSGPU_CUDA(cudaGetDevice(&dev));
-  if (device_needs_setup(g_lz_setup)) {
-    int nsm = 148, p0 = 0, p1 = 0;
-    MPSGPU_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    MPSGPU_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&p0, lanczos_step_kernel<false>, T, 0));
-    MPSGPU_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&p1, lanczos_step_kernel<true>, T, 0));
-    MPSGPU_CHECK(p0 >= 2 && p1 >= 2, MPSGPU_BAD_SHAPE, "lanczos step: kernel does not fit twice on an SM");
-    g_lz_sms[dev] = nsm;
-    mark_device_done(g_lz_setup);
-  }
-  const int nsm = g_lz_sms[dev], G = lz_max_ctas(nsm);
+  const int nsm = lz_setup(), G = lz_max_ctas(nsm);
   // the form with the basis in registers while every CTA slot's share is at
   // most 64 rows
   long long small = 0;
