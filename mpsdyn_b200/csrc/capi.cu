@@ -760,6 +760,9 @@ mpsgpu_status mpsgpu_heff_matvec(mpsgpu_context* ctx, const int* ldims, const do
   });
 }
 
+// Intermediate of a group of products kept in the context between calls: 256 MB.
+static constexpr long long kGroupKeep = (256LL << 20) / sizeof(cplx);
+
 mpsgpu_status mpsgpu_heff_matvec_grouped_ex(mpsgpu_context* ctx, int n, const mpsgpu_heff_instance* inst,
                                             int precision, int repeats, double* ms_per_run, double* flops,
                                             double* ms_prepare) {
@@ -774,15 +777,18 @@ mpsgpu_status mpsgpu_heff_matvec_grouped_ex(mpsgpu_context* ctx, int n, const mp
       v[i].L = (const cplx*)s.L; v[i].W = (const cplx*)s.W; v[i].Rt = (const cplx*)s.Rt;
       v[i].x = (const cplx*)s.x; v[i].y = (cplx*)s.y;
     }
-    int nsm = 148;
-    MPSGPU_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c.device));
-    GroupedMatvecPlan plan;
     const Stream st = c.st();
     const bool split = precision == 1;
-    grouped_matvec_plan(st, v, plan, nsm, split);
-    const int per_run = split ? 6 : 4;  // launches of one grouped product
+    GroupedMatvecPlan plan;
+    HeffGroup group;
+    auto release = [&]() {
+      if (split) grouped_matvec_free(st, plan);
+      // the intermediate of a large group goes back; a small one stays for the next call
+      else if (c.gws.cap > kGroupKeep) dbuf_free(c, c.gws);
+    };
     try {
       if (split) {
+        grouped_matvec_plan(st, v, plan);
         MPSGPU_CUDA(cudaEventRecord(c.mv0, c.stream));
         grouped_matvec_prepare_env(st, plan);
         MPSGPU_CUDA(cudaEventRecord(c.mv1, c.stream));
@@ -790,18 +796,25 @@ mpsgpu_status mpsgpu_heff_matvec_grouped_ex(mpsgpu_context* ctx, int n, const mp
         float ms = 0.f;
         MPSGPU_CUDA(cudaEventElapsedTime(&ms, c.mv0, c.mv1));
         if (ms_prepare) *ms_prepare = ms;
-      } else if (ms_prepare) {
-        *ms_prepare = 0.0;
+      } else {
+        heff_group_plan(c, v, group);
+        if (ms_prepare) *ms_prepare = 0.0;
       }
-      grouped_matvec_run(st, plan);
-      if (flops) *flops = plan.flops;
+      auto run = [&](const Stream& s) {
+        if (split) grouped_matvec_run(s, plan);
+        else heff_group_run(c, s, group);
+      };
+      run(st);
+      if (flops) *flops = split ? plan.flops : group.flops;
       if (repeats > 0) {
+        const int per_run = split ? 6 : group.launches();  // launches of one grouped product
         cudaGraph_t graph = nullptr;
         cudaGraphExec_t exec = nullptr;
         Stream cap = st;
         cap.launches = nullptr;  // the captured launches are counted per replay below
+        cap.prof = nullptr;      // no profiler events inside a graph
         MPSGPU_CUDA(cudaStreamBeginCapture(c.stream, cudaStreamCaptureModeThreadLocal));
-        grouped_matvec_run(cap, plan);
+        run(cap);
         MPSGPU_CUDA(cudaStreamEndCapture(c.stream, &graph));
         MPSGPU_CUDA(cudaGraphInstantiate(&exec, graph, 0));
         MPSGPU_CUDA(cudaGraphLaunch(exec, c.stream));  // warm replay
@@ -823,11 +836,11 @@ mpsgpu_status mpsgpu_heff_matvec_grouped_ex(mpsgpu_context* ctx, int n, const mp
         MPSGPU_CHECK(herr == 0, MPSGPU_TIMEOUT, "grouped matvec: a bounded wait in the tensor-core kernel ran out");
       }
     } catch (...) {
-      grouped_matvec_free(st, plan);
+      release();
       throw;
     }
-    grouped_matvec_free(st, plan);
-    MPSGPU_CUDA(cudaStreamSynchronize(c.stream));
+    release();
+    if (split) MPSGPU_CUDA(cudaStreamSynchronize(c.stream));
   });
 }
 

@@ -621,6 +621,61 @@ void heff_apply_hermitian(Context& c, const cplx* Le, const cplx* Lh, const std:
   }
 }
 
+void heff_group_plan(Context& c, const std::vector<HeffInstance>& inst, HeffGroup& g) {
+  const std::vector<int> order = grouped_matvec_order(inst);
+  const int n = (int)order.size();
+  long long n2 = 0;
+  for (const auto& h : inst) n2 += (long long)h.Dl * h.d * h.Dr * h.wr;
+  dbuf_reserve(c, c.gws, n2);
+  cplx* t2 = c.gws.p;
+  g.d1.clear();
+  g.d3.clear();
+  for (int i : order) {
+    const HeffInstance& h = inst[i];
+    Gemm1wDesc a = heff_first_desc(h.L, h.Dl, h.Dl, h.wl, h.x, h.d, h.Dr, h.W, h.d, h.wr, t2);
+    a.w_ref = 1;
+    g.d1.push_back(a);
+    g.d3.push_back(heff_last_desc(t2, h.Dl * h.d, h.Rt, h.Dr * h.wr, h.Dr, h.y, nullptr, make_double2(0.0, 0.0)));
+    t2 += (long long)h.Dl * h.d * h.Dr * h.wr;
+    g.flops += grouped_matvec_flops(h);
+  }
+  g.l1.clear();
+  g.l3.clear();
+  if (n <= GEMM_MAXP) return;
+  for (int q = 0; q < n; q += GEMM_MAXX) {
+    const int m = std::min(GEMM_MAXX, n - q);
+    g.l1.emplace_back();
+    heff_gemm1w_plan(&g.d1[q], m, g.l1.back());
+    g.l3.emplace_back();
+    heff_gemm3_plan(&g.d3[q], m, g.l3.back());
+  }
+  const size_t b1 = n * sizeof(Gemm1wDesc), b3 = n * sizeof(Gemm3Desc), off = (b1 + 15) & ~size_t(15);
+  uint8_t* d = bytes_reserve(c, c.gdesc, off + b3);
+  // (copies from pageable memory have left it when the calls return)
+  MPSGPU_CUDA(cudaMemcpyAsync(d, g.d1.data(), b1, cudaMemcpyHostToDevice, c.stream));
+  MPSGPU_CUDA(cudaMemcpyAsync(d + off, g.d3.data(), b3, cudaMemcpyHostToDevice, c.stream));
+}
+
+void heff_group_run(Context& c, const Stream& st, HeffGroup& g) {
+  const int n = (int)g.d1.size();
+  if (n <= GEMM_MAXP) {
+    Gemm1wBatch b1;
+    Gemm3Batch b3;
+    b1.n = b3.n = n;
+    std::copy(g.d1.begin(), g.d1.end(), b1.d);
+    std::copy(g.d3.begin(), g.d3.end(), b3.d);
+    heff_gemm1w(st, b1);
+    heff_gemm3(st, b3);
+    return;
+  }
+  const size_t off = (n * sizeof(Gemm1wDesc) + 15) & ~size_t(15);
+  const uint8_t* d = reinterpret_cast<const uint8_t*>(c.gdesc.p);
+  for (size_t i = 0; i < g.l1.size(); i++)
+    heff_gemm1w(st, g.l1[i], reinterpret_cast<const Gemm1wDesc*>(d) + i * GEMM_MAXX);
+  for (size_t i = 0; i < g.l3.size(); i++)
+    heff_gemm3(st, g.l3[i], reinterpret_cast<const Gemm3Desc*>(d + off) + i * GEMM_MAXX);
+}
+
 // Copies a descriptor blob into the next slot of the context's ring and
 // returns the slot's device address (the copy is ordered on c's stream before
 // the launches that read it).
@@ -1160,7 +1215,7 @@ void context_release(Context& c) {
   cudaSetDevice(c.device);
   for (auto& sc : c.subs) context_release(*sc);
   c.subs.clear();
-  for (DBuf* b : {&c.t1, &c.t2, &c.t3, &c.t4, &c.matA, &c.matQ, &c.matR, &c.lzws}) dbuf_free(c, *b);
+  for (DBuf* b : {&c.t1, &c.t2, &c.t3, &c.t4, &c.matA, &c.matQ, &c.matR, &c.lzws, &c.gws, &c.gdesc}) dbuf_free(c, *b);
   c.scratch.release();
   c.qrws.release();
   c.lzone.release(c);

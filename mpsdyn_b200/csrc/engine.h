@@ -76,6 +76,7 @@ struct Context {
   // reusable workspaces (complex elements)
   DBuf t1, t2, t3, t4, matA, matQ, matR;
   DBuf lzws;           // workspace of the fused Lanczos step (partial dots and norms)
+  DBuf gws, gdesc;     // intermediate and descriptors of a group of products
   LzWork lzone;        // eigensolver workspace of single solves
   int* hlz_err = nullptr;  // pinned, mapped: set when a grid barrier of the Lanczos step ran out
   int* dlz_err = nullptr;  // its device address
@@ -233,6 +234,19 @@ Gemm1wDesc heff_first_desc(const cplx* Le, int Dlb, int Dlk, int wl, const cplx*
                            int du, int wr, cplx* t2);
 Gemm3Desc heff_last_desc(const cplx* t2, int M, const cplx* Rt, int K, int Drb, cplx* y, const cplx* x,
                          cplx offset);
+// Grouped FP64 products of independent instances in device layouts: the two
+// contractions of every instance (the MPO tensors read as the reference stores
+// them), up to GEMM_MAXP instances with their descriptors as kernel parameters.
+// The descriptors and the intermediate live in the context until the next call.
+struct HeffGroup {
+  std::vector<Gemm1wDesc> d1;
+  std::vector<Gemm3Desc> d3;
+  std::vector<HeffLaunch> l1, l3;  // per GEMM_MAXX instances (more than GEMM_MAXP in all)
+  double flops = 0.0;
+  int launches() const { return l1.empty() ? 2 : 2 * (int)l1.size(); }
+};
+void heff_group_plan(Context& c, const std::vector<HeffInstance>& inst, HeffGroup& g);
+void heff_group_run(Context& c, const Stream& st, HeffGroup& g);
 // Left/right environment update (Operator::contractleftop / contractrightop).
 void env_left_update(Context& c, const cplx* Le, const std::array<int, 3>& ld, const MpsDev& ket,
                      const MpoDev* m, int k, const MpsDev& bra, DBuf& out,

@@ -1,10 +1,10 @@
-// Grouped effective-Hamiltonian matvec: y_i = L_i . W_i . R_i . x_i for many
-// independent instances of different shapes (bond dimensions, MPO bonds) in
-// three launches -- grouped GEMM (L.x), grouped MPO-leg contraction, grouped
-// GEMM (.R) -- each a persistent grid over the flattened tiles or pixels of
-// all instances.  The three launches can be captured once in a CUDA graph and
-// replayed.  Instances are scheduled largest first so that the tail of each
-// launch is filled by small tiles.
+// Grouped effective-Hamiltonian matvec in split precision: y_i = L_i . W_i .
+// R_i . x_i for many independent instances of different shapes (bond
+// dimensions, MPO bonds) in grouped launches -- limb planes, GEMM (L.x), MPO
+// legs, limb planes, GEMM (.R) -- over the flattened tiles or pixels of all
+// instances (the FP64 form runs the two contractions of heff.cu).  The launches
+// can be captured once in a CUDA graph and replayed.  Instances are scheduled
+// largest first so that the tail of each launch is filled by small tiles.
 #include <algorithm>
 #include <numeric>
 #include <vector>
@@ -131,21 +131,29 @@ void wcontract_grouped(const Stream& st, const WGroup* d_wg, int n, long long pi
   after_launch(st);
 }
 
-GroupedMatvecPlan::~GroupedMatvecPlan() {}
-
-void grouped_matvec_plan(const Stream& st, const std::vector<HeffInstance>& inst, GroupedMatvecPlan& plan,
-                         int nsm, bool split) {
+std::vector<int> grouped_matvec_order(const std::vector<HeffInstance>& inst) {
   const int n = (int)inst.size();
   MPSGPU_CHECK(n > 0, MPSGPU_INVALID, "grouped matvec: no instances");
-  // largest first
+  for (const auto& h : inst)
+    MPSGPU_CHECK(h.d > 0 && h.wl > 0 && h.wr > 0 && h.Dl > 0 && h.Dr > 0 && h.d * h.wl <= 32 && h.d * h.wr <= 32,
+                 MPSGPU_BAD_SHAPE, "grouped matvec: bad instance shape");
   std::vector<int> order(n);
   std::iota(order.begin(), order.end(), 0);
   auto work = [&](int i) { return (double)inst[i].Dl * inst[i].Dr * (inst[i].Dl + inst[i].Dr) * inst[i].wl; };
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return work(a) > work(b); });
+  return order;
+}
+
+double grouped_matvec_flops(const HeffInstance& h) {
+  return 8.0 * ((double)h.Dl * h.wl * h.Dl * h.d * h.Dr + (double)h.Dl * h.d * h.d * h.wl * h.wr * h.Dr +
+                (double)h.Dl * h.d * h.Dr * h.wr * h.Dr);
+}
+
+void grouped_matvec_plan(const Stream& st, const std::vector<HeffInstance>& inst, GroupedMatvecPlan& plan) {
+  const int n = (int)inst.size();
+  const std::vector<int> order = grouped_matvec_order(inst);
   long long t1_total = 0, wm_total = 0, pix_total = 0, wel_total = 0;
   for (const auto& h : inst) {
-    MPSGPU_CHECK(h.d > 0 && h.wl > 0 && h.wr > 0 && h.Dl > 0 && h.Dr > 0 && h.d * h.wl <= 32 && h.d * h.wr <= 32,
-                 MPSGPU_BAD_SHAPE, "grouped matvec: bad instance shape");
     t1_total += (long long)h.Dl * h.wl * h.d * h.Dr;
     wm_total += (long long)h.d * h.wl * h.d * h.wr;
     pix_total += (long long)h.Dl * h.Dr;
@@ -155,12 +163,11 @@ void grouped_matvec_plan(const Stream& st, const std::vector<HeffInstance>& inst
   dbuf_alloc(st, plan.t1, t1_total);
   dbuf_alloc(st, plan.t2, t1_total);
   dbuf_alloc(st, plan.wm, wm_total);
-  std::vector<GroupedGemm> g1(n), g3(n);
   std::vector<WGroup> wg(n);
   std::vector<WPerm> wp(n);
-  // split form: byte offsets of every prepared operand in one buffer
-  std::vector<SplitProblem> s1(split ? n : 0), s3(split ? n : 0);
-  std::vector<SplitPrepJob> jenv(split ? 2 * n : 0), jx(split ? n : 0), jt(split ? n : 0);
+  // byte offsets of every prepared operand in one buffer
+  std::vector<SplitProblem> s1(n), s3(n);
+  std::vector<SplitPrepJob> jenv(2 * n), jx(n), jt(n);
   std::vector<long long> offL(n), offX(n), offT(n), offR(n);
   long long spb = 0;
   auto take = [&](long long bytes) {
@@ -178,11 +185,6 @@ void grouped_matvec_plan(const Stream& st, const std::vector<HeffInstance>& inst
     cplx* T2 = plan.t2.p + o1;
     cplx* Wm = plan.wm.p + ow;
     wp[q] = WPerm{h.W, Wm, d, wl, d, wr, ow};
-    GroupedGemm& a = g1[q];
-    a.M = Dl * wl; a.N = d * Dr; a.K = Dl;
-    a.A = h.L; a.lda = (long long)Dl * wl;
-    a.B = h.x; a.ldb = Dl;
-    a.C = T1; a.ldc = (long long)Dl * wl;
     WContractArgs& w = wg[q].a;
     w.nx = Dl; w.ny = Dr;
     w.in = T1; w.ix = 1; w.iy = (long long)Dl * wl * d; w.si0 = Dl; w.si1 = (long long)Dl * wl;
@@ -191,92 +193,73 @@ void grouped_matvec_plan(const Stream& st, const std::vector<HeffInstance>& inst
     w.n_o0 = d; w.n_o1 = wr;
     w.Wm = Wm;
     wg[q].pix_begin = pix;
-    GroupedGemm& b = g3[q];
-    b.M = Dl * d; b.N = Dr; b.K = Dr * wr;
-    b.A = T2; b.lda = (long long)Dl * d;
-    b.B = h.Rt; b.ldb = (long long)Dr * wr;
-    b.C = h.y; b.ldc = (long long)Dl * d;
     o1 += (long long)Dl * wl * d * Dr;
     ow += (long long)d * wl * d * wr;
     pix += wcontract_chunked((long long)Dl * Dr);
     maxnin = std::max(maxnin, wl * d);
     maxnout = std::max(maxnout, d * wr);
-    if (split) {
-      offL[q] = take(split_operand_bytes(Dl * wl, Dl, 128));
-      offX[q] = take(split_operand_bytes(d * Dr, Dl, 128));
-      offT[q] = take(split_operand_bytes(Dl * d, Dr * wr, 128));
-      offR[q] = take(split_operand_bytes(Dr, Dr * wr, 128));
-      // L as A (rows Dl*wl), x as B (rows = columns of T1), T2 as A, Rt as B
-      jenv[2 * q] = SplitPrepJob{Dl * wl, Dl, 0, h.L, 1, (long long)Dl * wl, nullptr, 0};
-      jenv[2 * q + 1] = SplitPrepJob{Dr, Dr * wr, 0, h.Rt, (long long)Dr * wr, 1, nullptr, 0};
-      jx[q] = SplitPrepJob{d * Dr, Dl, 0, h.x, Dl, 1, nullptr, 0};
-      jt[q] = SplitPrepJob{Dl * d, Dr * wr, 0, T2, 1, (long long)Dl * d, nullptr, 0};
-      s1[q].M = Dl * wl; s1[q].N = d * Dr; s1[q].K = Dl;
-      s1[q].C = T1; s1[q].ldc = (long long)Dl * wl;
-      s3[q].M = Dl * d; s3[q].N = Dr; s3[q].K = Dr * wr;
-      s3[q].C = h.y; s3[q].ldc = (long long)Dl * d;
-    }
-    plan.flops += 8.0 * ((double)Dl * wl * Dl * d * Dr + (double)Dl * d * d * wl * wr * Dr +
-                         (double)Dl * d * Dr * wr * Dr);
+    offL[q] = take(split_operand_bytes(Dl * wl, Dl, 128));
+    offX[q] = take(split_operand_bytes(d * Dr, Dl, 128));
+    offT[q] = take(split_operand_bytes(Dl * d, Dr * wr, 128));
+    offR[q] = take(split_operand_bytes(Dr, Dr * wr, 128));
+    // L as A (rows Dl*wl), x as B (rows = columns of T1), T2 as A, Rt as B
+    jenv[2 * q] = SplitPrepJob{Dl * wl, Dl, 0, h.L, 1, (long long)Dl * wl, nullptr, 0};
+    jenv[2 * q + 1] = SplitPrepJob{Dr, Dr * wr, 0, h.Rt, (long long)Dr * wr, 1, nullptr, 0};
+    jx[q] = SplitPrepJob{d * Dr, Dl, 0, h.x, Dl, 1, nullptr, 0};
+    jt[q] = SplitPrepJob{Dl * d, Dr * wr, 0, T2, 1, (long long)Dl * d, nullptr, 0};
+    s1[q].M = Dl * wl; s1[q].N = d * Dr; s1[q].K = Dl;
+    s1[q].C = T1; s1[q].ldc = (long long)Dl * wl;
+    s3[q].M = Dl * d; s3[q].N = Dr; s3[q].K = Dr * wr;
+    s3[q].C = h.y; s3[q].ldc = (long long)Dl * d;
+    plan.flops += grouped_matvec_flops(h);
   }
-  plan.tiles1 = grouped_tiles(g1.data(), n);
-  plan.tiles3 = grouped_tiles(g3.data(), n);
   plan.pixels = pix;
   plan.wel = wel_total;
   plan.maxnin = maxnin;
   plan.maxnout = maxnout;
   // descriptor tables in device memory
-  const size_t bytes = n * (2 * sizeof(GroupedGemm) + sizeof(WGroup) + sizeof(WPerm));
+  const size_t bytes = n * (sizeof(WGroup) + sizeof(WPerm));
   MPSGPU_CUDA(cudaMallocAsync(&plan.desc, bytes, st.s));
   char* p = (char*)plan.desc;
-  plan.d_g1 = (GroupedGemm*)p; p += n * sizeof(GroupedGemm);
-  plan.d_g3 = (GroupedGemm*)p; p += n * sizeof(GroupedGemm);
   plan.d_wg = p; p += n * sizeof(WGroup);
   plan.d_wp = p;
-  MPSGPU_CUDA(cudaMemcpyAsync(plan.d_g1, g1.data(), n * sizeof(GroupedGemm), cudaMemcpyHostToDevice, st.s));
-  MPSGPU_CUDA(cudaMemcpyAsync(plan.d_g3, g3.data(), n * sizeof(GroupedGemm), cudaMemcpyHostToDevice, st.s));
   MPSGPU_CUDA(cudaMemcpyAsync(plan.d_wg, wg.data(), n * sizeof(WGroup), cudaMemcpyHostToDevice, st.s));
   MPSGPU_CUDA(cudaMemcpyAsync(plan.d_wp, wp.data(), n * sizeof(WPerm), cudaMemcpyHostToDevice, st.s));
   MPSGPU_CUDA(cudaStreamSynchronize(st.s));
-  plan.ctas = nsm;
-  plan.split = split;
-  if (split) {
-    dbuf_alloc(st, plan.sp, (spb + (long long)sizeof(cplx) - 1) / (long long)sizeof(cplx));
-    uint8_t* base = reinterpret_cast<uint8_t*>(plan.sp.p);
-    for (int q = 0; q < n; q++) {
-      jenv[2 * q].out = base + offL[q];
-      jenv[2 * q + 1].out = base + offR[q];
-      jx[q].out = base + offX[q];
-      jt[q].out = base + offT[q];
-      s1[q].Ap = base + offL[q]; s1[q].Bp = base + offX[q];
-      s3[q].Ap = base + offT[q]; s3[q].Bp = base + offR[q];
-    }
-    plan.stiles1 = split_group_tiles(s1.data(), n);
-    plan.stiles3 = split_group_tiles(s3.data(), n);
-    plan.thr_env = split_prepare_jobs(jenv.data(), 2 * n);
-    plan.thr_x = split_prepare_jobs(jx.data(), n);
-    plan.thr_t = split_prepare_jobs(jt.data(), n);
-    const size_t sbytes = 2 * n * sizeof(SplitProblem) + 4 * n * sizeof(SplitPrepJob) + 256;
-    MPSGPU_CUDA(cudaMallocAsync(&plan.sdesc, sbytes, st.s));
-    char* sq = (char*)plan.sdesc;
-    plan.d_s1 = (SplitProblem*)sq; sq += n * sizeof(SplitProblem);
-    plan.d_s3 = (SplitProblem*)sq; sq += n * sizeof(SplitProblem);
-    plan.d_jenv = (SplitPrepJob*)sq; sq += 2 * n * sizeof(SplitPrepJob);
-    plan.d_jx = (SplitPrepJob*)sq; sq += n * sizeof(SplitPrepJob);
-    plan.d_jt = (SplitPrepJob*)sq; sq += n * sizeof(SplitPrepJob);
-    plan.err = (int*)sq;
-    MPSGPU_CUDA(cudaMemcpyAsync(plan.d_s1, s1.data(), n * sizeof(SplitProblem), cudaMemcpyHostToDevice, st.s));
-    MPSGPU_CUDA(cudaMemcpyAsync(plan.d_s3, s3.data(), n * sizeof(SplitProblem), cudaMemcpyHostToDevice, st.s));
-    MPSGPU_CUDA(cudaMemcpyAsync(plan.d_jenv, jenv.data(), 2 * n * sizeof(SplitPrepJob), cudaMemcpyHostToDevice, st.s));
-    MPSGPU_CUDA(cudaMemcpyAsync(plan.d_jx, jx.data(), n * sizeof(SplitPrepJob), cudaMemcpyHostToDevice, st.s));
-    MPSGPU_CUDA(cudaMemcpyAsync(plan.d_jt, jt.data(), n * sizeof(SplitPrepJob), cudaMemcpyHostToDevice, st.s));
-    MPSGPU_CUDA(cudaMemsetAsync(plan.err, 0, sizeof(int), st.s));
-    MPSGPU_CUDA(cudaStreamSynchronize(st.s));
+  dbuf_alloc(st, plan.sp, (spb + (long long)sizeof(cplx) - 1) / (long long)sizeof(cplx));
+  uint8_t* base = reinterpret_cast<uint8_t*>(plan.sp.p);
+  for (int q = 0; q < n; q++) {
+    jenv[2 * q].out = base + offL[q];
+    jenv[2 * q + 1].out = base + offR[q];
+    jx[q].out = base + offX[q];
+    jt[q].out = base + offT[q];
+    s1[q].Ap = base + offL[q]; s1[q].Bp = base + offX[q];
+    s3[q].Ap = base + offT[q]; s3[q].Bp = base + offR[q];
   }
+  plan.stiles1 = split_group_tiles(s1.data(), n);
+  plan.stiles3 = split_group_tiles(s3.data(), n);
+  plan.thr_env = split_prepare_jobs(jenv.data(), 2 * n);
+  plan.thr_x = split_prepare_jobs(jx.data(), n);
+  plan.thr_t = split_prepare_jobs(jt.data(), n);
+  const size_t sbytes = 2 * n * sizeof(SplitProblem) + 4 * n * sizeof(SplitPrepJob) + 256;
+  MPSGPU_CUDA(cudaMallocAsync(&plan.sdesc, sbytes, st.s));
+  char* sq = (char*)plan.sdesc;
+  plan.d_s1 = (SplitProblem*)sq; sq += n * sizeof(SplitProblem);
+  plan.d_s3 = (SplitProblem*)sq; sq += n * sizeof(SplitProblem);
+  plan.d_jenv = (SplitPrepJob*)sq; sq += 2 * n * sizeof(SplitPrepJob);
+  plan.d_jx = (SplitPrepJob*)sq; sq += n * sizeof(SplitPrepJob);
+  plan.d_jt = (SplitPrepJob*)sq; sq += n * sizeof(SplitPrepJob);
+  plan.err = (int*)sq;
+  MPSGPU_CUDA(cudaMemcpyAsync(plan.d_s1, s1.data(), n * sizeof(SplitProblem), cudaMemcpyHostToDevice, st.s));
+  MPSGPU_CUDA(cudaMemcpyAsync(plan.d_s3, s3.data(), n * sizeof(SplitProblem), cudaMemcpyHostToDevice, st.s));
+  MPSGPU_CUDA(cudaMemcpyAsync(plan.d_jenv, jenv.data(), 2 * n * sizeof(SplitPrepJob), cudaMemcpyHostToDevice, st.s));
+  MPSGPU_CUDA(cudaMemcpyAsync(plan.d_jx, jx.data(), n * sizeof(SplitPrepJob), cudaMemcpyHostToDevice, st.s));
+  MPSGPU_CUDA(cudaMemcpyAsync(plan.d_jt, jt.data(), n * sizeof(SplitPrepJob), cudaMemcpyHostToDevice, st.s));
+  MPSGPU_CUDA(cudaMemsetAsync(plan.err, 0, sizeof(int), st.s));
+  MPSGPU_CUDA(cudaStreamSynchronize(st.s));
 }
 
 void grouped_matvec_prepare_env(const Stream& st, GroupedMatvecPlan& plan) {
-  MPSGPU_CHECK(plan.split, MPSGPU_INVALID, "grouped matvec: not planned in split precision");
   split_prepare_grouped(st, plan.d_jenv, 2 * plan.n, plan.thr_env);
 }
 
@@ -285,19 +268,11 @@ void grouped_matvec_run(const Stream& st, GroupedMatvecPlan& plan) {
   wperm_kernel<<<std::min<long long>(ceil_div(plan.wel, 256), 4096), 256, 0, st.s>>>(
       (const WPerm*)plan.d_wp, plan.n, plan.wel);
   after_launch(st);
-  if (plan.split) {
-    split_prepare_grouped(st, plan.d_jx, plan.n, plan.thr_x);
-    zgemm_split_grouped(st, plan.d_s1, plan.n, plan.stiles1, plan.err);
-  } else {
-    zgemm_grouped(st, plan.d_g1, plan.n, plan.tiles1, plan.ctas);
-  }
+  split_prepare_grouped(st, plan.d_jx, plan.n, plan.thr_x);
+  zgemm_split_grouped(st, plan.d_s1, plan.n, plan.stiles1, plan.err);
   wcontract_grouped(st, (const WGroup*)plan.d_wg, plan.n, plan.pixels, plan.maxnin, plan.maxnout);
-  if (plan.split) {
-    split_prepare_grouped(st, plan.d_jt, plan.n, plan.thr_t);
-    zgemm_split_grouped(st, plan.d_s3, plan.n, plan.stiles3, plan.err);
-  } else {
-    zgemm_grouped(st, plan.d_g3, plan.n, plan.tiles3, plan.ctas);
-  }
+  split_prepare_grouped(st, plan.d_jt, plan.n, plan.thr_t);
+  zgemm_split_grouped(st, plan.d_s3, plan.n, plan.stiles3, plan.err);
 }
 
 void grouped_matvec_free(const Stream& st, GroupedMatvecPlan& plan) {

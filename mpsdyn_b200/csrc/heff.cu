@@ -194,24 +194,61 @@ __device__ __forceinline__ void acc_to_smem(const Acc<BM, BN, NS>& acc, cplx* Cs
   }
 }
 
-// tile t -> problem index (descriptors hold consecutive tile ranges)
+// Descriptors of a launch (consecutive tile ranges): up to GEMM_MAXP as kernel
+// parameters, up to GEMM_MAXX in device memory, with the tile ranges as
+// parameters (the search reads constant memory) and the tile's descriptor
+// copied to shared memory.
 template <class D>
-__device__ __forceinline__ int problem_of(const D* d, int n, int t) {
-  int q = 0;
-  while (q + 1 < n && d[q + 1].tile_begin <= t) q++;
-  return q;
-}
+struct Extern {
+  int n;
+  const D* d;
+  int tile_begin[GEMM_MAXX];
+};
+template <class B>
+struct Source;
+template <class D, class B>
+struct ParamSource {
+  using Desc = D;
+  struct Slot {};
+  static __device__ __forceinline__ const D& pick(const B& b, int t, Slot&) {
+    int q = 0;
+    while (q + 1 < b.n && b.d[q + 1].tile_begin <= t) q++;
+    return b.d[q];
+  }
+};
+template <>
+struct Source<Gemm1wBatch> : ParamSource<Gemm1wDesc, Gemm1wBatch> {};
+template <>
+struct Source<Gemm3Batch> : ParamSource<Gemm3Desc, Gemm3Batch> {};
+template <class D>
+struct Source<Extern<D>> {
+  using Desc = D;
+  using Slot = D;
+  static __device__ __forceinline__ const D& pick(const Extern<D>& b, int t, Slot& slot) {
+    int lo = 0, hi = b.n - 1;
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (b.tile_begin[mid] <= t) lo = mid;
+      else hi = mid - 1;
+    }
+    const int* src = reinterpret_cast<const int*>(b.d + lo);
+    for (int e = threadIdx.x; e < (int)(sizeof(D) / sizeof(int)); e += blockDim.x)
+      reinterpret_cast<int*>(&slot)[e] = src[e];
+    __syncthreads();
+    return slot;
+  }
+};
 
 // ---------------------------------------------------------------------------
 // heff_gemm1w
 // ---------------------------------------------------------------------------
-template <int BM, int BN, int NS>
-__global__ void __launch_bounds__(nthreads<BM>(), BM <= 32 ? 3 : 2) heff_gemm1w_kernel(const __grid_constant__ Gemm1wBatch b) {
+template <int BM, int BN, int NS, class B>
+__global__ void __launch_bounds__(nthreads<BM>(), BM <= 32 ? 3 : 2) heff_gemm1w_kernel(const __grid_constant__ B b) {
+  __shared__ typename Source<B>::Slot slot;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int NT_ = nthreads<BM>();
   Ring<BM, BN>& ring = *reinterpret_cast<Ring<BM, BN>*>(smem_raw);
-  const int q = problem_of(b.d, b.n, blockIdx.x);
-  const Gemm1wDesc& d = b.d[q];
+  const Gemm1wDesc& d = Source<B>::pick(b, blockIdx.x, slot);
   const int local = blockIdx.x - d.tile_begin;
   const int TX = BM / d.n_i0, TY = BN / d.n_i1;
   const int tx = local % d.tiles_x, ty = local / d.tiles_x;
@@ -264,7 +301,16 @@ __global__ void __launch_bounds__(nthreads<BM>(), BM <= 32 ? 3 : 2) heff_gemm1w_
   const cplx* Wp = d.Wm;
   if (nw <= (int)((ring_bytes<BM, BN>() - BM * LD * sizeof(cplx)) / sizeof(cplx))) {
     cplx* Ws = Cs + BM * LD;
-    for (int e = tid; e < nw; e += NT_) Ws[e] = __ldg(&d.Wm[e]);
+    for (int e = tid; e < nw; e += NT_) {
+      int to = e;
+      if (d.w_ref) {  // W(o0, i0, i1, o1)
+        int r = e;
+        const int o0 = r % d.n_o0; r /= d.n_o0;
+        const int i0 = r % d.n_i0; r /= d.n_i0;
+        to = o0 + d.n_o0 * (r / d.n_i1) + nout * (i0 + d.n_i0 * (r % d.n_i1));
+      }
+      Ws[to] = __ldg(&d.Wm[e]);
+    }
     Wp = Ws;
   }
   acc_to_smem<BM, BN, NS>(acc, Cs);
@@ -300,15 +346,15 @@ __global__ void __launch_bounds__(nthreads<BM>(), BM <= 32 ? 3 : 2) heff_gemm1w_
 // ---------------------------------------------------------------------------
 // heff_gemm3 (cluster split-K)
 // ---------------------------------------------------------------------------
-template <int BM, int BN, int CS, int NS>
+template <int BM, int BN, int CS, int NS, class B>
 __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(nthreads<BM>(), BM <= 32 ? 3 : 2)
-    heff_gemm3_kernel(const __grid_constant__ Gemm3Batch b) {
+    heff_gemm3_kernel(const __grid_constant__ B b) {
+  __shared__ typename Source<B>::Slot slot;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int NT_ = nthreads<BM>();
   Ring<BM, BN>& ring = *reinterpret_cast<Ring<BM, BN>*>(smem_raw);
   const int tile = blockIdx.x / CS, rank = blockIdx.x % CS;
-  const int q = problem_of(b.d, b.n, tile);
-  const Gemm3Desc& d = b.d[q];
+  const Gemm3Desc& d = Source<B>::pick(b, tile, slot);
   const int local = tile - d.tile_begin;
   const int tm = local % d.tiles_m, tn = local / d.tiles_m;
   const int m0 = tm * BM, n0 = tn * BN;
@@ -396,21 +442,32 @@ void set_smem(K kernel, size_t bytes) {
   MPSGPU_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
 }
 
+template <class B>
+void heff_setup1() {
+  set_smem(heff_gemm1w_kernel<64, 32, 2, B>, ring_bytes<64, 32>());
+  set_smem(heff_gemm1w_kernel<32, 32, 2, B>, ring_bytes<32, 32>());
+  set_smem(heff_gemm1w_kernel<32, 32, 4, B>, ring_bytes<32, 32>());
+}
+template <class B>
+void heff_setup3() {
+  set_smem(heff_gemm3_kernel<64, 32, 1, 2, B>, ring_bytes<64, 32>());
+  set_smem(heff_gemm3_kernel<32, 32, 1, 4, B>, ring_bytes<32, 32>());
+  set_smem(heff_gemm3_kernel<32, 32, 1, 2, B>, ring_bytes<32, 32>());
+  set_smem(heff_gemm3_kernel<32, 32, 2, 2, B>, ring_bytes<32, 32>());
+  set_smem(heff_gemm3_kernel<32, 32, 4, 2, B>, ring_bytes<32, 32>());
+  set_smem(heff_gemm3_kernel<32, 32, 8, 2, B>, ring_bytes<32, 32>());
+}
+
 std::atomic<unsigned long long> g_heff_setup{0};
 std::mutex g_heff_mu;
 
 void heff_setup() {
   if (!device_needs_setup(g_heff_setup)) return;
   std::lock_guard<std::mutex> lk(g_heff_mu);
-  set_smem(heff_gemm1w_kernel<64, 32, 2>, ring_bytes<64, 32>());
-  set_smem(heff_gemm1w_kernel<32, 32, 2>, ring_bytes<32, 32>());
-  set_smem(heff_gemm1w_kernel<32, 32, 4>, ring_bytes<32, 32>());
-  set_smem(heff_gemm3_kernel<64, 32, 1, 2>, ring_bytes<64, 32>());
-  set_smem(heff_gemm3_kernel<32, 32, 1, 4>, ring_bytes<32, 32>());
-  set_smem(heff_gemm3_kernel<32, 32, 1, 2>, ring_bytes<32, 32>());
-  set_smem(heff_gemm3_kernel<32, 32, 2, 2>, ring_bytes<32, 32>());
-  set_smem(heff_gemm3_kernel<32, 32, 4, 2>, ring_bytes<32, 32>());
-  set_smem(heff_gemm3_kernel<32, 32, 8, 2>, ring_bytes<32, 32>());
+  heff_setup1<Gemm1wBatch>();
+  heff_setup1<Extern<Gemm1wDesc>>();
+  heff_setup3<Gemm3Batch>();
+  heff_setup3<Extern<Gemm3Desc>>();
   mark_device_done(g_heff_setup);
 }
 
@@ -427,66 +484,83 @@ int sm_count() {
   return v;
 }
 
-}  // namespace
-
-void heff_gemm1w(const Stream& st, Gemm1wBatch& b) {
-  MPSGPU_CHECK(b.n >= 1 && b.n <= GEMM_MAXP, MPSGPU_BAD_SHAPE, "gemm1w: group size");
-  heff_setup();
-  // tile rows: 32 (two warp groups splitting the k steps, twice the warps per
-  // SM), measured faster for the grouped products of lockstep batches of 8
-  // chains at D = 128 as well as for one chain; 64 only for groups that fill
-  // the GPU many times over
-  long long t64 = 0;
-  bool single = true;  // every problem one 16 x 16 tile of pixels at most
-  for (int q = 0; q < b.n; q++) {
-    const Gemm1wDesc& d = b.d[q];
-    single = single && d.X <= 16 && d.Y <= 16;
-    MPSGPU_CHECK(d.n_i0 >= 1 && d.n_i0 <= 32 && d.n_i1 >= 1 && d.n_i1 <= 32 && d.X > 0 && d.Y > 0 && d.K > 0,
-                 MPSGPU_BAD_SHAPE, "gemm1w: leg dimensions");
-    t64 += (long long)ceil_div(d.X, 64 / d.n_i0) * ceil_div(d.Y, 32 / d.n_i1);
-  }
-  const int bm = t64 >= 16LL * sm_count() ? 64 : 32;
-  int tiles = 0;
-  for (int q = 0; q < b.n; q++) {
-    Gemm1wDesc& d = b.d[q];
-    MPSGPU_CHECK(bm / d.n_i0 >= 1 && 32 / d.n_i1 >= 1, MPSGPU_BAD_SHAPE, "gemm1w: MPO legs wider than a tile");
-    d.tiles_x = ceil_div(d.X, bm / d.n_i0);
-    d.tiles_y = ceil_div(d.Y, 32 / d.n_i1);
-    d.tile_begin = tiles;
-    tiles += d.tiles_x * d.tiles_y;
-  }
-  double work = 0.0;  // GEMM flops plus the MPO-leg epilogue
-  for (int q = 0; q < b.n; q++) {
-    const Gemm1wDesc& d = b.d[q];
-    const double nin = (double)d.n_i0 * d.n_i1, nout = (double)d.n_o0 * d.n_o1;
-    work += 8.0 * ((double)d.X * d.n_i0 * d.Y * d.n_i1 * d.K + (double)d.X * d.Y * nout * nin);
-  }
-  ProfScope ps(st, GemmProfiler::GEMM64, work);
-  if (bm == 64)
-    heff_gemm1w_kernel<64, 32, 2><<<tiles, nthreads<64>(), ring_bytes<64, 32>(), st.s>>>(b);
-  else if (single)
-    heff_gemm1w_kernel<32, 32, 4><<<tiles, nthreads<32>(), ring_bytes<32, 32>(), st.s>>>(b);
+template <class B>
+void launch1(const Stream& st, const HeffLaunch& l, const B& b) {
+  ProfScope ps(st, GemmProfiler::GEMM64, l.work);
+  if (l.bm == 64)
+    heff_gemm1w_kernel<64, 32, 2><<<l.tiles, nthreads<64>(), ring_bytes<64, 32>(), st.s>>>(b);
+  else if (l.single)
+    heff_gemm1w_kernel<32, 32, 4><<<l.tiles, nthreads<32>(), ring_bytes<32, 32>(), st.s>>>(b);
   else
-    heff_gemm1w_kernel<32, 32, 2><<<tiles, nthreads<32>(), ring_bytes<32, 32>(), st.s>>>(b);
+    heff_gemm1w_kernel<32, 32, 2><<<l.tiles, nthreads<32>(), ring_bytes<32, 32>(), st.s>>>(b);
   after_launch(st);
 }
 
-void heff_gemm3(const Stream& st, Gemm3Batch& b) {
-  MPSGPU_CHECK(b.n >= 1 && b.n <= GEMM_MAXP, MPSGPU_BAD_SHAPE, "gemm3: group size");
-  heff_setup();
+template <class B>
+void launch3(const Stream& st, const HeffLaunch& l, const B& b) {
+  ProfScope ps(st, GemmProfiler::GEMM64, l.work);
+  const dim3 grid(l.tiles * l.cs);
+#define MPSGPU_G3(BMv, CSv, NSv) \
+  heff_gemm3_kernel<BMv, 32, CSv, NSv><<<grid, nthreads<BMv>(), ring_bytes<BMv, 32>(), st.s>>>(b)
+  if (l.bm == 64) {
+    MPSGPU_G3(64, 1, 2);
+  } else if (l.single) {
+    MPSGPU_G3(32, 1, 4);
+  } else if (l.cs == 1) {
+    MPSGPU_G3(32, 1, 2);
+  } else if (l.cs == 2) {
+    MPSGPU_G3(32, 2, 2);
+  } else if (l.cs == 4) {
+    MPSGPU_G3(32, 4, 2);
+  } else {
+    MPSGPU_G3(32, 8, 2);
+  }
+#undef MPSGPU_G3
+  after_launch(st);
+}
+
+// tile ranges and launch shape of a group of first contractions
+void plan1(Gemm1wDesc* d, int n, HeffLaunch& l) {
+  // tile rows: 32 (two warp groups splitting the k steps), measured faster for
+  // the grouped products of lockstep batches of 8 chains at D = 128 as well as
+  // for one chain; 64 only for groups that fill the GPU many times over
+  long long t64 = 0;
+  l.n = n;
+  l.single = true;  // every problem one 16 x 16 tile of pixels at most
+  for (int q = 0; q < n; q++) {
+    l.single = l.single && d[q].X <= 16 && d[q].Y <= 16;
+    MPSGPU_CHECK(d[q].n_i0 >= 1 && d[q].n_i0 <= 32 && d[q].n_i1 >= 1 && d[q].n_i1 <= 32 && d[q].X > 0 && d[q].Y > 0 &&
+                     d[q].K > 0 &&
+                     (!d[q].w_ref || d[q].n_i0 * d[q].n_i1 * d[q].n_o0 * d[q].n_o1 <= GEMM_WREF),
+                 MPSGPU_BAD_SHAPE, "gemm1w: leg dimensions");
+    t64 += (long long)ceil_div(d[q].X, 64 / d[q].n_i0) * ceil_div(d[q].Y, 32 / d[q].n_i1);
+  }
+  l.bm = t64 >= 16LL * sm_count() ? 64 : 32;
+  l.tiles = 0;
+  l.work = 0.0;  // GEMM flops plus the MPO-leg epilogue
+  for (int q = 0; q < n; q++) {
+    MPSGPU_CHECK(l.bm / d[q].n_i0 >= 1 && 32 / d[q].n_i1 >= 1, MPSGPU_BAD_SHAPE, "gemm1w: MPO legs wider than a tile");
+    d[q].tiles_x = ceil_div(d[q].X, l.bm / d[q].n_i0);
+    d[q].tiles_y = ceil_div(d[q].Y, 32 / d[q].n_i1);
+    d[q].tile_begin = l.tiles;
+    l.tiles += d[q].tiles_x * d[q].tiles_y;
+    const double nin = (double)d[q].n_i0 * d[q].n_i1, nout = (double)d[q].n_o0 * d[q].n_o1;
+    l.work += 8.0 * ((double)d[q].X * d[q].n_i0 * d[q].Y * d[q].n_i1 * d[q].K + (double)d[q].X * d[q].Y * nout * nin);
+  }
+}
+
+void plan3(Gemm3Desc* d, int n, HeffLaunch& l) {
   const int nsm = sm_count();
-  // tile rows and split-K: the largest K chunk that still gives about one
-  // CTA per SM
   long long t64 = 0, t32 = 0;
   int kmax = 0;
-  bool single = true;  // every problem at most one tile of a D = 16 site
-  for (int q = 0; q < b.n; q++) {
-    const Gemm3Desc& d = b.d[q];
-    single = single && d.M <= 32 && d.N <= 16;
-    MPSGPU_CHECK(d.M > 0 && d.N > 0 && d.K1 > 0 && d.K2 >= 0, MPSGPU_BAD_SHAPE, "gemm3: shape");
-    t64 += (long long)ceil_div(d.M, 64) * ceil_div(d.N, 32);
-    t32 += (long long)ceil_div(d.M, 32) * ceil_div(d.N, 32);
-    kmax = std::max(kmax, d.K1 + d.K2);
+  l.n = n;
+  l.single = true;  // every problem at most one tile of a D = 16 site
+  for (int q = 0; q < n; q++) {
+    l.single = l.single && d[q].M <= 32 && d[q].N <= 16;
+    MPSGPU_CHECK(d[q].M > 0 && d[q].N > 0 && d[q].K1 > 0 && d[q].K2 >= 0, MPSGPU_BAD_SHAPE, "gemm3: shape");
+    t64 += (long long)ceil_div(d[q].M, 64) * ceil_div(d[q].N, 32);
+    t32 += (long long)ceil_div(d[q].M, 32) * ceil_div(d[q].N, 32);
+    kmax = std::max(kmax, d[q].K1 + d[q].K2);
   }
   // 64-row tiles (two CTAs per SM by shared memory) once they alone fill the
   // GPU twice; otherwise 32-row tiles, with the K range split over a cluster
@@ -494,40 +568,66 @@ void heff_gemm3(const Stream& st, Gemm3Batch& b) {
   // do not pack the SMs of a GPC to the last one: at 576 CTAs in clusters of 8
   // a third wave took 38 us where 288 in clusters of 4 take 33 us) and K chunks
   // of at least four slabs
-  int bm = 64, cs = 1;
+  l.bm = 64;
+  l.cs = 1;
   if (t64 < 2LL * nsm) {
-    bm = 32;
-    while (!single && cs < 8 && t32 * cs * 2 <= 2LL * nsm && kmax / (cs * 2) >= 4 * BK) cs *= 2;
+    l.bm = 32;
+    while (!l.single && l.cs < 8 && t32 * l.cs * 2 <= 2LL * nsm && kmax / (l.cs * 2) >= 4 * BK) l.cs *= 2;
   }
-  int tiles = 0;
-  for (int q = 0; q < b.n; q++) {
-    Gemm3Desc& d = b.d[q];
-    d.tiles_m = ceil_div(d.M, bm);
-    d.tiles_n = ceil_div(d.N, 32);
-    d.tile_begin = tiles;
-    tiles += d.tiles_m * d.tiles_n;
+  l.tiles = 0;
+  l.work = 0.0;
+  for (int q = 0; q < n; q++) {
+    d[q].tiles_m = ceil_div(d[q].M, l.bm);
+    d[q].tiles_n = ceil_div(d[q].N, 32);
+    d[q].tile_begin = l.tiles;
+    l.tiles += d[q].tiles_m * d[q].tiles_n;
+    l.work += 8.0 * (double)d[q].M * d[q].N * (d[q].K1 + d[q].K2);
   }
-  const dim3 grid(tiles * cs);
-  double work = 0.0;
-  for (int q = 0; q < b.n; q++) work += 8.0 * (double)b.d[q].M * b.d[q].N * (b.d[q].K1 + b.d[q].K2);
-  ProfScope ps(st, GemmProfiler::GEMM64, work);
-#define MPSGPU_G3(BMv, CSv, NSv)                                                                   \
-  heff_gemm3_kernel<BMv, 32, CSv, NSv><<<grid, nthreads<BMv>(), ring_bytes<BMv, 32>(), st.s>>>(b)
-  if (bm == 64) {
-    MPSGPU_G3(64, 1, 2);
-  } else if (single) {
-    MPSGPU_G3(32, 1, 4);
-  } else if (cs == 1) {
-    MPSGPU_G3(32, 1, 2);
-  } else if (cs == 2) {
-    MPSGPU_G3(32, 2, 2);
-  } else if (cs == 4) {
-    MPSGPU_G3(32, 4, 2);
-  } else {
-    MPSGPU_G3(32, 8, 2);
-  }
-#undef MPSGPU_G3
-  after_launch(st);
+}
+
+template <class D>
+Extern<D> external(const HeffLaunch& l, const D* dev) {
+  Extern<D> e;
+  e.n = l.n;
+  e.d = dev;
+  std::copy(l.tile_begin, l.tile_begin + l.n, e.tile_begin);
+  return e;
+}
+
+}  // namespace
+
+void heff_gemm1w(const Stream& st, Gemm1wBatch& b) {
+  MPSGPU_CHECK(b.n >= 1 && b.n <= GEMM_MAXP, MPSGPU_BAD_SHAPE, "gemm1w: group size");
+  heff_setup();
+  HeffLaunch l;
+  plan1(b.d, b.n, l);
+  launch1(st, l, b);
+}
+void heff_gemm1w_plan(Gemm1wDesc* d, int n, HeffLaunch& l) {
+  MPSGPU_CHECK(n >= 1 && n <= GEMM_MAXX, MPSGPU_BAD_SHAPE, "gemm1w: group size");
+  plan1(d, n, l);
+  for (int q = 0; q < n; q++) l.tile_begin[q] = d[q].tile_begin;
+}
+void heff_gemm1w(const Stream& st, const HeffLaunch& l, const Gemm1wDesc* dev) {
+  heff_setup();
+  launch1(st, l, external(l, dev));
+}
+
+void heff_gemm3(const Stream& st, Gemm3Batch& b) {
+  MPSGPU_CHECK(b.n >= 1 && b.n <= GEMM_MAXP, MPSGPU_BAD_SHAPE, "gemm3: group size");
+  heff_setup();
+  HeffLaunch l;
+  plan3(b.d, b.n, l);
+  launch3(st, l, b);
+}
+void heff_gemm3_plan(Gemm3Desc* d, int n, HeffLaunch& l) {
+  MPSGPU_CHECK(n >= 1 && n <= GEMM_MAXX, MPSGPU_BAD_SHAPE, "gemm3: group size");
+  plan3(d, n, l);
+  for (int q = 0; q < n; q++) l.tile_begin[q] = d[q].tile_begin;
+}
+void heff_gemm3(const Stream& st, const HeffLaunch& l, const Gemm3Desc* dev) {
+  heff_setup();
+  launch3(st, l, external(l, dev));
 }
 
 }  // namespace mpsgpu

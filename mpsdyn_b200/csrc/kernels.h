@@ -51,21 +51,6 @@ void set_gemm_autotune(int on);
 long long gemm_autotune_entries();
 bool gemm_autotune_on();
 
-// One GEMM C = A B (op N, N) of a grouped launch; tile_begin / tiles_m are
-// filled by grouped_tiles (64 x 64 tiles).
-struct GroupedGemm {
-  int M = 0, N = 0, K = 0;
-  const cplx* A = nullptr; long long lda = 0;
-  const cplx* B = nullptr; long long ldb = 0;
-  cplx* C = nullptr; long long ldc = 0;
-  long long tile_begin = 0;
-  int tiles_m = 0;
-};
-// Host: assigns tile ranges in order; returns the total number of tiles.
-long long grouped_tiles(GroupedGemm* descs, int n);
-// All tiles of n GEMMs (descriptors in device memory) in one persistent launch of `ctas` CTAs.
-void zgemm_grouped(const Stream& st, const GroupedGemm* d_descs, int n, long long total_tiles, int ctas);
-
 // ---- split-precision complex GEMM (umma.cu): BF16 limbs on tcgen05 ----
 // Tiling of C = A B (M x N, inner K): 128-row A tiles, BN-column B tiles,
 // k-steps of 16, K split over `splits` CTAs of ks_per_split k-steps each.
@@ -153,20 +138,18 @@ inline void dbuf_alloc(const Stream& st, DevMem& m, long long n) {
   MPSGPU_CUDA(cudaMallocAsync((void**)&m.p, std::max<long long>(n, 1) * sizeof(cplx), st.s));
   m.n = n;
 }
+// Split-precision plan of a group (tcgen05, BF16 limbs).
 struct GroupedMatvecPlan {
   int n = 0;
   DevMem t1, t2, wm;
   void* desc = nullptr;
-  GroupedGemm* d_g1 = nullptr;
-  GroupedGemm* d_g3 = nullptr;
   void* d_wg = nullptr;
   void* d_wp = nullptr;
-  long long tiles1 = 0, tiles3 = 0, pixels = 0, wel = 0;
-  int maxnin = 1, maxnout = 1, ctas = 148;
+  long long pixels = 0, wel = 0;
+  int maxnin = 1, maxnout = 1;
   double flops = 0.0;  // algorithmic flops of one grouped product
-  // split precision: BF16 limb planes of L, Rt (prepared once by
-  // grouped_matvec_prepare_env), x and T2 (prepared in every product)
-  bool split = false;
+  // BF16 limb planes of L, Rt (prepared once by grouped_matvec_prepare_env), x
+  // and T2 (prepared in every product)
   DevMem sp;                                  // all prepared planes
   void* sdesc = nullptr;                      // device tables below
   SplitProblem* d_s1 = nullptr;               // T1 = L . x
@@ -176,15 +159,16 @@ struct GroupedMatvecPlan {
   SplitPrepJob* d_jt = nullptr;               // T2, n jobs
   long long stiles1 = 0, stiles3 = 0, thr_env = 0, thr_x = 0, thr_t = 0;
   int* err = nullptr;                         // set by a tensor-core kernel whose bounded wait ran out
-  ~GroupedMatvecPlan();
 };
-// split = true plans the split-precision form (tcgen05, BF16 limbs).
-void grouped_matvec_plan(const Stream& st, const std::vector<HeffInstance>& inst, GroupedMatvecPlan& plan,
-                         int nsm, bool split = false);
-// Split form: the limb planes of the environments, made once per set of instances.
+void grouped_matvec_plan(const Stream& st, const std::vector<HeffInstance>& inst, GroupedMatvecPlan& plan);
+// The limb planes of the environments, made once per set of instances.
 void grouped_matvec_prepare_env(const Stream& st, GroupedMatvecPlan& plan);
 void grouped_matvec_run(const Stream& st, GroupedMatvecPlan& plan);
 void grouped_matvec_free(const Stream& st, GroupedMatvecPlan& plan);
+// Instances in descending order of their work (the tail of a launch is then
+// filled by small tiles), their shapes checked.
+std::vector<int> grouped_matvec_order(const std::vector<HeffInstance>& inst);
+double grouped_matvec_flops(const HeffInstance& h);
 
 // MPO-leg contraction: for every pixel (x, y) in [0,nx) x [0,ny)
 //   out[x*ox + y*oy + o0*so0 + o1*so1] =
@@ -229,15 +213,29 @@ struct Gemm1wDesc {
   long long ldb = 0;
   int X = 0, Y = 0, K = 0, n_i0 = 0, n_i1 = 0, n_o0 = 0, n_o1 = 0;
   const cplx* Wm = nullptr;
+  int w_ref = 0;  // Wm is the MPO tensor as the reference stores it, W(o0, i0, i1, o1) (nin nout <= GEMM_WREF)
   cplx* out = nullptr;
   long long ox = 0, oy = 0, so0 = 0, so1 = 0;
   int tiles_x = 0, tiles_y = 0, tile_begin = 0;  // filled by heff_gemm1w
 };
+constexpr int GEMM_WREF = 1024;
 struct Gemm1wBatch {
   int n = 0;
   Gemm1wDesc d[GEMM_MAXP];
 };
 void heff_gemm1w(const Stream& st, Gemm1wBatch& b);
+// The same for up to GEMM_MAXX problems whose descriptors lie in device
+// memory: plan fills the tile fields of the host copies (before they are
+// copied over) and chooses the launch, which reads `dev`.
+constexpr int GEMM_MAXX = 192;
+struct HeffLaunch {
+  int n = 0, bm = 32, cs = 1, tiles = 0;
+  bool single = false;
+  double work = 0.0;
+  int tile_begin[GEMM_MAXX];
+};
+void heff_gemm1w_plan(Gemm1wDesc* d, int n, HeffLaunch& l);
+void heff_gemm1w(const Stream& st, const HeffLaunch& l, const Gemm1wDesc* dev);
 // C = alpha (A1 B1 + A2 B2) + beta Cin, column-major, op N: A1 M x K1,
 // B1 K1 x N, and (K2 > 0) A2 M x K2, B2 K2 x N; Cin may be null.
 struct Gemm3Desc {
@@ -262,6 +260,8 @@ struct Gemm3Batch {
   Gemm3Desc d[GEMM_MAXP];
 };
 void heff_gemm3(const Stream& st, Gemm3Batch& b);
+void heff_gemm3_plan(Gemm3Desc* d, int n, HeffLaunch& l);
+void heff_gemm3(const Stream& st, const HeffLaunch& l, const Gemm3Desc* dev);
 
 // ---- vector kernels (Lanczos, norms) ----
 // dots[j] = sum_i conj(V[i + j*ldv]) w[i], j < k   (two-stage, deterministic)

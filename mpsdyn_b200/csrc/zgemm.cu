@@ -18,9 +18,7 @@
 // (padded rows: conflict-free fragment loads); the next K-slab is prefetched
 // into registers while the current one is consumed.  Large-K, small-MN
 // problems are split over K into a workspace and reduced by a second kernel
-// that also applies the epilogue (deterministic order).  A grouped variant
-// runs the tiles of many independent GEMMs (different shapes) in one
-// persistent launch.
+// that also applies the epilogue (deterministic order).
 #include <atomic>
 #include <cstdlib>
 #include <map>
@@ -218,31 +216,6 @@ zgemm_dmma_kernel(GemmArgs g, int splits, int kchunk, cplx* __restrict__ partial
   }
 }
 
-// Grouped GEMMs (op N, N): descriptor d covers tiles [tile_begin(d), tile_begin(d+1)).
-template <int BM, int BN, int WMW, int WNW>
-__global__ void __launch_bounds__(WMW* WNW * 32)
-zgemm_grouped_kernel(const GroupedGemm* __restrict__ descs, int ndesc, long long total_tiles) {
-  __shared__ TileSmem<BM, BN> sm;
-  double acc[BM / WMW / 8][BN / WNW / 8][4][2];
-  for (long long t = blockIdx.x; t < total_tiles; t += gridDim.x) {
-    // binary search for the descriptor owning tile t
-    int lo = 0, hi = ndesc - 1;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (descs[mid].tile_begin <= t) lo = mid;
-      else hi = mid - 1;
-    }
-    const GroupedGemm& d = descs[lo];
-    const long long local = t - d.tile_begin;
-    const int tm = (int)(local % d.tiles_m), tn = (int)(local / d.tiles_m);
-    const int m0 = tm * BM, n0 = tn * BN;
-    gemm_tile<BM, BN, WMW, WNW, OP_N, OP_N>(d.A, d.lda, d.B, d.ldb, d.M, d.N, m0, n0, 0, d.K, sm, acc);
-    tile_store<BM, BN, WMW, WNW>(acc, d.M, d.N, m0, n0, make_double2(1.0, 0.0), nullptr, 0,
-                                 make_double2(0.0, 0.0), d.C, d.ldc, false);
-    __syncthreads();
-  }
-}
-
 __global__ void splitk_reduce_kernel(GemmArgs g, int splits, const cplx* __restrict__ partial) {
   long long mn = (long long)g.M * g.N;
   long long total = mn * g.batch;
@@ -433,23 +406,6 @@ void zgemm(const Stream& st, const GemmArgs& g0, Scratch& scratch) {
   const GemmCfg cfg = choose_cfg(st, g, scratch);
   ProfScope ps(st, GemmProfiler::GEMM64, 8.0 * (double)g.M * g.N * g.K * g.batch);
   run_cfg(st, g, cfg, scratch);
-}
-
-long long grouped_tiles(GroupedGemm* descs, int n) {
-  long long t = 0;
-  for (int i = 0; i < n; i++) {
-    descs[i].tiles_m = ceil_div(descs[i].M, 64);
-    const int tiles_n = ceil_div(descs[i].N, 64);
-    descs[i].tile_begin = t;
-    t += (long long)descs[i].tiles_m * tiles_n;
-  }
-  return t;
-}
-
-void zgemm_grouped(const Stream& st, const GroupedGemm* d_descs, int n, long long total_tiles, int ctas) {
-  if (n <= 0 || total_tiles <= 0) return;
-  zgemm_grouped_kernel<64, 64, 2, 4><<<ctas, 256, 0, st.s>>>(d_descs, n, total_tiles);
-  after_launch(st);
 }
 
 }  // namespace mpsgpu
