@@ -28,14 +28,17 @@
 // re.im, im.re): they are bound by the latency of one tile, and the chain of
 // dependent DMMAs (27 cycles each) is half as long.
 //
-// Bound by the FP64 tensor pipe (a DMMA per 4 cycles and SM) once a group has
-// tiles for every SM, by latency below.  Around the main loop, the epilogue of
-// heff_gemm1w took three times its instructions while it divided by the leg
-// dimensions for every term; it now walks the legs with the leg matrix staged
-// in the ring's space.  Measured: four Hermitian products (eight problems) at
-// D = 96, w = 5 in 30.6 us for the first contraction and 33.3 us for the last one
-// (38.4 us with clusters of 8), one product at D = 64, w = 3 in 9.0 and 10.0 us
-// (9.8 and 10.7 us).
+// Bound by the FP64 tensor pipe (a DMMA per 4 cycles and SM, 36.8 TF) once a
+// group has tiles for every SM, by latency below.  Around the main loop:
+//   - a thread keeps two running addresses per operand and an early-out per
+//     slab instead of recomputing rows, columns and edges for every copy
+//     (gemm3, eight problems at D = 96: 31.3 us -> 28.9 us);
+//   - the leg epilogue is itself a product, pixels x legs, on the DMMA from
+//     shared memory with offsets in tables; as scalar code it took 25 us of the
+//     84 us of eight problems at D = 128, w = 5, now 8 us of 67 us.
+// Measured now: D = 128, w = 5, eight problems 67 and 57 us (20 and 23.5 TF), one
+// 20.6 and 14.5 us; D = 64, w = 3, one 10.3 and 8.3 us; D = 400, w = 3, four 446
+// and 440 us (28 TF).
 #include <cooperative_groups.h>
 
 #include <mutex>
@@ -67,10 +70,9 @@ __device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b)
                : "d"(a), "d"(b));
 }
 
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem, bool valid) {
-  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+__device__ __forceinline__ void cp_async16(unsigned smem, const void* gmem, bool valid) {
   const int n = valid ? 16 : 0;
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(n));
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem), "l"(gmem), "r"(n));
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 template <int N>
@@ -96,11 +98,81 @@ struct Acc {
   double v[MT][NT][NS][2];
 };
 
-// Main loop over k in [kbeg, kend): loadA(ring, stage, k0) / loadB(...)
-// issue the cp.async copies of one BK slab.
-template <int BM, int BN, int NS, class LA, class LB>
-__device__ __forceinline__ void mainloop(Ring<BM, BN>& r, Acc<BM, BN, NS>& acc, int kbeg, int kend, LA loadA,
-                                         LB loadB) {
+// The copies a thread makes of every slab: a column of the A slab (one row,
+// AE values of k) and BE columns of the B slab at one k.  The addresses step by
+// constants from slab to slab; only a slab that K ends in tests k.
+template <int BM, int BN>
+struct Feed {
+  static constexpr int NT_ = nthreads<BM>(), AK = NT_ / BM, BC = NT_ / BK;
+  static constexpr int AE = BK / AK, BE = BN / BC;
+  const cplx *pa, *pb;          // the thread's first entries of the next slab
+  long long ua, ub;             // between its entries
+  long long sa;                 // of A per slab (B: BK)
+  const cplx *base_a, *base_b;  // any valid address, for copies that read nothing
+  unsigned da, db;              // shared addresses in stage 0
+  bool oka;
+  unsigned okb;                 // per column
+
+  // row: the thread's row of A (offset arow, negative: outside); ncols: columns of the tile inside
+  __device__ __forceinline__ void start(Ring<BM, BN>& r, const cplx* A, long long lda, long long arow, const cplx* B,
+                                        long long ldb, int ncols) {
+    const int tid = threadIdx.x, mt = tid % BM, ka = tid / BM, kb = tid % BK, nt = tid / BK;
+    da = (unsigned)__cvta_generic_to_shared(&r.A[0][ka][mt]);
+    db = (unsigned)__cvta_generic_to_shared(&r.B[0][kb][nt]);
+    oka = arow >= 0;
+    okb = 0;
+#pragma unroll
+    for (int u = 0; u < BE; u++) okb |= (nt + u * BC < ncols ? 1u : 0u) << u;
+    source(A, lda, arow, B, ldb);
+  }
+  __device__ __forceinline__ void source(const cplx* A, long long lda, long long arow, const cplx* B, long long ldb) {
+    const int tid = threadIdx.x;
+    base_a = A;
+    base_b = B;
+    ua = AK * lda;
+    sa = BK * lda;
+    pa = A + (oka ? arow : 0) + (tid / BM) * lda;
+    ub = BC * ldb;
+    pb = B + tid % BK + (long long)(tid / BK) * ldb;
+  }
+  __device__ __forceinline__ void skip(int slabs) {
+    pa += slabs * sa;
+    pb += (long long)slabs * BK;
+  }
+  // the next slab into a stage; left: values of k it still holds
+  __device__ __forceinline__ void issue(int stage, int left) {
+    const unsigned a = da + stage * (unsigned)(BK * (BM + PADC) * sizeof(cplx));
+    const unsigned b = db + stage * (unsigned)(BK * (BN + PADC) * sizeof(cplx));
+    constexpr unsigned astep = AK * (BM + PADC) * sizeof(cplx), bstep = BC * sizeof(cplx);
+    if (left >= BK) {
+#pragma unroll
+      for (int u = 0; u < AE; u++) cp_async16(a + u * astep, oka ? pa + u * ua : base_a, oka);
+#pragma unroll
+      for (int u = 0; u < BE; u++) {
+        const bool ok = (okb >> u) & 1;
+        cp_async16(b + u * bstep, ok ? pb + u * ub : base_b, ok);
+      }
+    } else {
+      const int ka = threadIdx.x / BM, kb = threadIdx.x % BK;
+#pragma unroll
+      for (int u = 0; u < AE; u++) {
+        const bool ok = oka && ka + u * AK < left;
+        cp_async16(a + u * astep, ok ? pa + u * ua : base_a, ok);
+      }
+#pragma unroll
+      for (int u = 0; u < BE; u++) {
+        const bool ok = ((okb >> u) & 1) && kb < left;
+        cp_async16(b + u * bstep, ok ? pb + u * ub : base_b, ok);
+      }
+    }
+    pa += sa;
+    pb += BK;
+  }
+};
+
+// Main loop over nslab slabs: issue(stage, slab) copies one.
+template <int BM, int BN, int NS, class Issue>
+__device__ __forceinline__ void mainloop(Ring<BM, BN>& r, Acc<BM, BN, NS>& acc, int nslab, Issue issue) {
   using AC = Acc<BM, BN, NS>;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int wm0 = (warp & 1) * AC::WM, wn0 = ((warp >> 1) & 1) * AC::WN, kg = warp >> 2;
@@ -111,25 +183,18 @@ __device__ __forceinline__ void mainloop(Ring<BM, BN>& r, Acc<BM, BN, NS>& acc, 
     for (int j = 0; j < AC::NT; j++)
 #pragma unroll
       for (int s = 0; s < NS; s++) acc.v[i][j][s][0] = acc.v[i][j][s][1] = 0.0;
-  const int nslab = kend > kbeg ? (kend - kbeg + BK - 1) / BK : 0;
 #pragma unroll
   for (int s = 0; s < STAGES - 1; s++) {
-    if (s < nslab) {
-      loadA(r, s, kbeg + s * BK);
-      loadB(r, s, kbeg + s * BK);
-    }
+    if (s < nslab) issue(s, s);
     cp_async_commit();
   }
+  int st = 0, fill = STAGES - 1;  // stages: computed on, filled
   for (int it = 0; it < nslab; it++) {
     cp_async_wait<STAGES - 2>();
     __syncthreads();
-    const int nx = it + STAGES - 1;
-    if (nx < nslab) {
-      loadA(r, nx % STAGES, kbeg + nx * BK);
-      loadB(r, nx % STAGES, kbeg + nx * BK);
-    }
+    if (it + STAGES - 1 < nslab) issue(fill, it + STAGES - 1);
     cp_async_commit();
-    const int st = it % STAGES;
+    fill = fill + 1 == STAGES ? 0 : fill + 1;
 #pragma unroll
     for (int kk0 = 0; kk0 < BK; kk0 += 4 * kgroups<BM>()) {
       const int kk = kk0 + 4 * kg;  // this group's k step of the slab
@@ -158,6 +223,7 @@ __device__ __forceinline__ void mainloop(Ring<BM, BN>& r, Acc<BM, BN, NS>& acc, 
           dmma(acc.v[i][j][IR][0], acc.v[i][j][IR][1], aim[i], bre[j]);
         }
     }
+    st = st + 1 == STAGES ? 0 : st + 1;
   }
   cp_async_wait<0>();
   __syncthreads();
@@ -254,70 +320,81 @@ __global__ void __launch_bounds__(nthreads<BM>(), BM <= 32 ? 3 : 2) heff_gemm1w_
   const int tx = local % d.tiles_x, ty = local / d.tiles_x;
   const int x0 = tx * TX, y0 = ty * TY;
   const int tid = threadIdx.x;
-  // the (row, k) and (k, column) slots this thread copies are the same in
-  // every slab: their row/column offsets are computed once (-1 = outside)
-  constexpr int AE = BM * BK / NT_, BE = BN * BK / NT_;
-  long long aoff[AE], boff[BE];
-#pragma unroll
-  for (int u = 0; u < AE; u++) {
-    const int mt = (tid + u * NT_) % BM;
-    const int xl = mt % TX, i0 = mt / TX, x = x0 + xl;
-    aoff[u] = (i0 < d.n_i0 && x < d.X) ? x + (long long)d.X * i0 : -1;
-  }
+  long long arow;
   {
-    const int ncols = min(TY, d.Y - y0) * d.n_i1;
-#pragma unroll
-    for (int u = 0; u < BE; u++) {
-      const int nt = (tid + u * NT_) / BK;
-      boff[u] = nt < ncols ? ((long long)d.n_i1 * y0 + nt) * d.ldb : -1;
-    }
+    const int mt = tid % BM, xl = mt % TX, i0 = mt / TX, x = x0 + xl;
+    arow = (i0 < d.n_i0 && x < d.X) ? x + (long long)d.X * i0 : -1;
   }
-  auto loadA = [&](Ring<BM, BN>& r, int st, int k0) {
-#pragma unroll
-    for (int u = 0; u < AE; u++) {
-      const int e = tid + u * NT_;
-      const int mt = e % BM, kk = e / BM;
-      const int k = k0 + kk;
-      const bool ok = aoff[u] >= 0 && k < d.K;
-      cp_async16(&r.A[st][kk][mt], ok ? d.A + aoff[u] + (long long)k * d.lda : d.A, ok);
-    }
-  };
-  auto loadB = [&](Ring<BM, BN>& r, int st, int k0) {
-#pragma unroll
-    for (int u = 0; u < BE; u++) {
-      const int e = tid + u * NT_;
-      const int kk = e % BK, nt = e / BK;
-      const int k = k0 + kk;
-      const bool ok = boff[u] >= 0 && k < d.K;
-      cp_async16(&r.B[st][kk][nt], ok ? d.B + k + boff[u] : d.B, ok);
-    }
-  };
+  Feed<BM, BN> feed;
+  feed.start(ring, d.A, d.lda, arow, d.B + (long long)d.n_i1 * y0 * d.ldb, d.ldb, min(TY, d.Y - y0) * d.n_i1);
   Acc<BM, BN, NS> acc;
-  mainloop<BM, BN, NS>(ring, acc, 0, d.K, loadA, loadB);
+  mainloop<BM, BN, NS>(ring, acc, (d.K + BK - 1) / BK, [&](int stage, int slab) { feed.issue(stage, d.K - slab * BK); });
   cplx* Cs = reinterpret_cast<cplx*>(smem_raw);
   constexpr int LD = BN + PADC;
-  // the leg matrix behind the tile, where the ring leaves room for it
-  const int nout = d.n_o0 * d.n_o1, nw = d.n_i0 * d.n_i1 * nout;
-  const cplx* Wp = d.Wm;
-  if (nw <= (int)((ring_bytes<BM, BN>() - BM * LD * sizeof(cplx)) / sizeof(cplx))) {
+  constexpr int ROOM = (int)(ring_bytes<BM, BN>() - BM * LD * sizeof(cplx));  // behind the tile
+  const int nin = d.n_i0 * d.n_i1, nout = d.n_o0 * d.n_o1, nw = nin * nout, npix = TX * TY;
+  // index of leg matrix element e (as stored) in an (i, o) order with o ld apart 1, i apart ld
+  auto leg_index = [&](int e, int ld) {
+    if (!d.w_ref) return e % nout + ld * (e / nout);
+    int r = e;  // W(o0, i0, i1, o1)
+    const int o0 = r % d.n_o0; r /= d.n_o0;
+    const int i0 = r % d.n_i0; r /= d.n_i0;
+    return o0 + d.n_o0 * (r / d.n_i1) + ld * (i0 + d.n_i0 * (r % d.n_i1));
+  };
+  // per pixel (x, y): out[o0 + n_o0 o1] = sum_{i0, i1} Wm[o, i0 + n_i0 i1] C[(x, i0), (i1, y)]
+  const int kp = (nin + 3) & ~3, no8 = (nout + 7) / 8, np8 = (npix + 7) / 8, wld = 8 * no8 + 2;
+  if (NS == 2 && kp * wld * (int)sizeof(cplx) + 20 * npix + 8 * nout + 8 * kp <= ROOM) {
+    // on the tensor pipe: pixels x legs in times legs in x legs out, 8 x 8 tiles
+    // over the warps; offsets of pixels and legs in tables
     cplx* Ws = Cs + BM * LD;
-    for (int e = tid; e < nw; e += NT_) {
-      int to = e;
-      if (d.w_ref) {  // W(o0, i0, i1, o1)
-        int r = e;
-        const int o0 = r % d.n_o0; r /= d.n_o0;
-        const int i0 = r % d.n_i0; r /= d.n_i0;
-        to = o0 + d.n_o0 * (r / d.n_i1) + nout * (i0 + d.n_i0 * (r % d.n_i1));
-      }
-      Ws[to] = __ldg(&d.Wm[e]);
+    long long* goff = reinterpret_cast<long long*>(Ws + kp * wld);  // global, -1 outside
+    long long* ooff = goff + npix;
+    int* poff = reinterpret_cast<int*>(ooff + nout);
+    int* ioff = poff + npix;
+    for (int e = tid; e < kp * wld; e += NT_) Ws[e] = make_double2(0.0, 0.0);
+    for (int pix = tid; pix < npix; pix += NT_) {
+      const int xl = pix % TX, yl = pix / TX, x = x0 + xl, y = y0 + yl;
+      goff[pix] = (x < d.X && y < d.Y) ? x * d.ox + y * d.oy : -1;
+      poff[pix] = xl * LD + d.n_i1 * yl;
     }
+    for (int o = tid; o < nout; o += NT_) ooff[o] = (o % d.n_o0) * d.so0 + (o / d.n_o0) * d.so1;
+    for (int i = tid; i < kp; i += NT_) ioff[i] = i < nin ? TX * (i % d.n_i0) * LD + i / d.n_i0 : -1;
+    __syncthreads();
+    for (int e = tid; e < nw; e += NT_) Ws[leg_index(e, wld)] = __ldg(&d.Wm[e]);
+    acc_to_smem<BM, BN, NS>(acc, Cs);  // ends with a barrier
+    const int lane = tid & 31, fr = lane >> 2, fc = lane & 3;
+    for (int u = tid >> 5; u < np8 * no8; u += NT_ / 32) {
+      const int pix = (u % np8) * 8 + fr, o8 = (u / np8) * 8;
+      const cplx* cp = Cs + (pix < npix ? poff[pix] : 0);
+      double re[2] = {0.0, 0.0}, im[2] = {0.0, 0.0};
+      for (int i = fc; i < kp; i += 4) {
+        const int io = ioff[i];
+        const cplx a = io >= 0 ? cp[io] : make_double2(0.0, 0.0), w = Ws[i * wld + o8 + fr];
+        dmma(re[0], re[1], a.x, w.x);
+        dmma(im[0], im[1], a.x, w.y);
+        dmma(re[0], re[1], -a.y, w.y);
+        dmma(im[0], im[1], a.y, w.x);
+      }
+      const long long go = pix < npix ? goff[pix] : -1;
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const int o = o8 + 2 * fc + h;
+        if (go >= 0 && o < nout) d.out[go + ooff[o]] = make_double2(re[h], im[h]);
+      }
+    }
+    return;
+  }
+  // scalar form (single-tile problems, and legs whose tables do not fit): ng
+  // threads per pixel, each every ng-th output, two at a time
+  const cplx* Wp = d.Wm;
+  if (nw * (int)sizeof(cplx) <= ROOM) {
+    cplx* Ws = Cs + BM * LD;
+    for (int e = tid; e < nw; e += NT_) Ws[leg_index(e, nout)] = __ldg(&d.Wm[e]);
     Wp = Ws;
   }
   acc_to_smem<BM, BN, NS>(acc, Cs);
   __syncthreads();
-  // per pixel (x, y): out[o0 + n_o0 o1] = sum_{i0, i1} Wm[o, i0 + n_i0 i1] C[(x, i0), (i1, y)];
-  // ng threads per pixel, each every ng-th output, two at a time
-  const int npix = TX * TY, ng = max(1, NT_ / npix);
+  const int ng = max(1, NT_ / npix);
   for (int p = tid; p < npix * ng; p += NT_) {
     const int pix = p % npix, g = p / npix;
     const int xl = pix % TX, yl = pix / TX;
@@ -358,46 +435,27 @@ __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(nthreads<BM>(), BM 
   const int local = tile - d.tile_begin;
   const int tm = local % d.tiles_m, tn = local / d.tiles_m;
   const int m0 = tm * BM, n0 = tn * BN;
-  const int Ktot = d.K1 + d.K2;
-  const int chunk = ((Ktot + CS - 1) / CS + BK - 1) / BK * BK;
-  const int kbeg = min(Ktot, rank * chunk), kend = min(Ktot, kbeg + chunk);
+  // slabs of the two sources, dealt to the ranks in equal runs
+  const int n1 = (d.K1 + BK - 1) / BK, ns = n1 + (d.K2 + BK - 1) / BK;
+  const int chunk = (ns + CS - 1) / CS, s0 = min(ns, rank * chunk), s1 = min(ns, s0 + chunk);
   const int tid = threadIdx.x;
-  // the (row, k) and (k, column) slots this thread copies are the same in every
-  // slab: their rows and columns are tested once (-1 = outside)
-  constexpr int AE = BM * BK / NT_, BE = BN * BK / NT_;
-  int am[AE], bn[BE];
-#pragma unroll
-  for (int u = 0; u < AE; u++) {
-    const int m = m0 + (tid + u * NT_) % BM;
-    am[u] = m < d.M ? m : -1;
+  const int m = m0 + tid % BM;
+  const long long arow = m < d.M ? m : -1;
+  Feed<BM, BN> feed;
+  feed.start(ring, d.A1, d.lda1, arow, d.B1 + (long long)n0 * d.ldb1, d.ldb1, d.N - n0);
+  auto second = [&]() { feed.source(d.A2, d.lda2, arow, d.B2 + (long long)n0 * d.ldb2, d.ldb2); };
+  if (s0 <= n1) {
+    feed.skip(s0);
+  } else {
+    second();
+    feed.skip(s0 - n1);
   }
-#pragma unroll
-  for (int u = 0; u < BE; u++) {
-    const int n = n0 + (tid + u * NT_) / BK;
-    bn[u] = n < d.N ? n : -1;
-  }
-  auto loadA = [&](Ring<BM, BN>& r, int st, int k0) {
-#pragma unroll
-    for (int u = 0; u < AE; u++) {
-      const int e = tid + u * NT_, mt = e % BM, kk = e / BM, k = k0 + kk;
-      const bool ok = am[u] >= 0 && k < kend;
-      const cplx* src = d.A1;
-      if (ok) src = k < d.K1 ? d.A1 + am[u] + (long long)k * d.lda1 : d.A2 + am[u] + (long long)(k - d.K1) * d.lda2;
-      cp_async16(&r.A[st][kk][mt], src, ok);
-    }
-  };
-  auto loadB = [&](Ring<BM, BN>& r, int st, int k0) {
-#pragma unroll
-    for (int u = 0; u < BE; u++) {
-      const int e = tid + u * NT_, kk = e % BK, nt = e / BK, k = k0 + kk;
-      const bool ok = bn[u] >= 0 && k < kend;
-      const cplx* src = d.B1;
-      if (ok) src = k < d.K1 ? d.B1 + k + (long long)bn[u] * d.ldb1 : d.B2 + (k - d.K1) + (long long)bn[u] * d.ldb2;
-      cp_async16(&r.B[st][kk][nt], src, ok);
-    }
-  };
   Acc<BM, BN, NS> acc;
-  mainloop<BM, BN, NS>(ring, acc, kbeg, kend, loadA, loadB);
+  mainloop<BM, BN, NS>(ring, acc, s1 - s0, [&](int stage, int slab) {
+    const int sl = s0 + slab;
+    if (sl == n1) second();
+    feed.issue(stage, sl < n1 ? d.K1 - sl * BK : d.K2 - (sl - n1) * BK);
+  });
   cplx* Cs = reinterpret_cast<cplx*>(smem_raw);
   acc_to_smem<BM, BN, NS>(acc, Cs);
   // rows [r0, r1) of the tile are finished by this rank: the sum over the
@@ -451,6 +509,8 @@ void heff_setup1() {
 template <class B>
 void heff_setup3() {
   set_smem(heff_gemm3_kernel<64, 32, 1, 2, B>, ring_bytes<64, 32>());
+  set_smem(heff_gemm3_kernel<64, 32, 2, 2, B>, ring_bytes<64, 32>());
+  set_smem(heff_gemm3_kernel<64, 32, 4, 2, B>, ring_bytes<64, 32>());
   set_smem(heff_gemm3_kernel<32, 32, 1, 4, B>, ring_bytes<32, 32>());
   set_smem(heff_gemm3_kernel<32, 32, 1, 2, B>, ring_bytes<32, 32>());
   set_smem(heff_gemm3_kernel<32, 32, 2, 2, B>, ring_bytes<32, 32>());
@@ -502,8 +562,12 @@ void launch3(const Stream& st, const HeffLaunch& l, const B& b) {
   const dim3 grid(l.tiles * l.cs);
 #define MPSGPU_G3(BMv, CSv, NSv) \
   heff_gemm3_kernel<BMv, 32, CSv, NSv><<<grid, nthreads<BMv>(), ring_bytes<BMv, 32>(), st.s>>>(b)
-  if (l.bm == 64) {
+  if (l.bm == 64 && l.cs == 1) {
     MPSGPU_G3(64, 1, 2);
+  } else if (l.bm == 64 && l.cs == 2) {
+    MPSGPU_G3(64, 2, 2);
+  } else if (l.bm == 64) {
+    MPSGPU_G3(64, 4, 2);
   } else if (l.single) {
     MPSGPU_G3(32, 1, 4);
   } else if (l.cs == 1) {
@@ -521,9 +585,11 @@ void launch3(const Stream& st, const HeffLaunch& l, const B& b) {
 
 // tile ranges and launch shape of a group of first contractions
 void plan1(Gemm1wDesc* d, int n, HeffLaunch& l) {
-  // tile rows: 32 (two warp groups splitting the k steps), measured faster for
-  // the grouped products of lockstep batches of 8 chains at D = 128 as well as
-  // for one chain; 64 only for groups that fill the GPU many times over
+  // 64 tile rows (half the B traffic of 32) once those tiles fill every SM
+  // twice: eight problems at D = 128, w = 5 take 67 us against 72 us and at
+  // D = 96 38 us against 39 us.  Below that 32 rows, with twice the tiles and
+  // warps: four problems at D = 96 (192 tiles of 64 rows) take 23 us against
+  // 27 us, one at D = 256, w = 3 (208) 41 us against 51 us
   long long t64 = 0;
   l.n = n;
   l.single = true;  // every problem one 16 x 16 tile of pixels at most
@@ -535,7 +601,7 @@ void plan1(Gemm1wDesc* d, int n, HeffLaunch& l) {
                  MPSGPU_BAD_SHAPE, "gemm1w: leg dimensions");
     t64 += (long long)ceil_div(d[q].X, 64 / d[q].n_i0) * ceil_div(d[q].Y, 32 / d[q].n_i1);
   }
-  l.bm = t64 >= 16LL * sm_count() ? 64 : 32;
+  l.bm = t64 >= 2LL * sm_count() ? 64 : 32;
   l.tiles = 0;
   l.work = 0.0;  // GEMM flops plus the MPO-leg epilogue
   for (int q = 0; q < n; q++) {
@@ -562,17 +628,27 @@ void plan3(Gemm3Desc* d, int n, HeffLaunch& l) {
     t32 += (long long)ceil_div(d[q].M, 32) * ceil_div(d[q].N, 32);
     kmax = std::max(kmax, d[q].K1 + d[q].K2);
   }
-  // 64-row tiles (two CTAs per SM by shared memory) once they alone fill the
-  // GPU twice; otherwise 32-row tiles, with the K range split over a cluster
-  // while the CTAs keep within two per SM (three fit, but clusters of 4 and 8
-  // do not pack the SMs of a GPC to the last one: at 576 CTAs in clusters of 8
-  // a third wave took 38 us where 288 in clusters of 4 take 33 us) and K chunks
-  // of at least four slabs
+  // 64-row tiles (half the B traffic, two CTAs per SM by shared memory) where
+  // they fill the GPU twice, by themselves or with the K range split over
+  // clusters of 2 or 4, whose CTAs must come to between 3/2 and 7/4 of the
+  // SMs (clusters of 4 do not pack the SMs of a GPC to the last one): eight
+  // problems at D = 128, w = 5 in 57 us, against 65 us with 32 rows.  Otherwise
+  // 32 rows in clusters of 2 up to two CTAs per SM, of 4 and 8 up to one (four
+  // problems at D = 96: 144 CTAs in clusters of 2 take 19.6 us, 288 in clusters
+  // of 4 23.6 us).  A rank's share is at least two slabs (one problem at D = 64,
+  // w = 3, K = 192: clusters of 4 8.3 us, of 2 10.4 us).
   l.bm = 64;
   l.cs = 1;
   if (t64 < 2LL * nsm) {
-    l.bm = 32;
-    while (!l.single && l.cs < 8 && t32 * l.cs * 2 <= 2LL * nsm && kmax / (l.cs * 2) >= 4 * BK) l.cs *= 2;
+    const int room = kmax / (2 * BK);  // largest useful cluster
+    int c = 1;
+    while (c < 4 && 4 * t64 * c * 2 <= 7LL * nsm && c * 2 <= room) c *= 2;
+    if (!l.single && 2 * t64 * c >= 3LL * nsm) {
+      l.cs = c;
+    } else {
+      l.bm = 32;
+      while (!l.single && l.cs < 8 && t32 * l.cs * 2 <= (l.cs == 1 ? 2LL : 1LL) * nsm && l.cs * 2 <= room) l.cs *= 2;
+    }
   }
   l.tiles = 0;
   l.work = 0.0;
