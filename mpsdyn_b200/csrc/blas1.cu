@@ -100,6 +100,7 @@ constexpr int DOT_CHUNK = 4096;
 // partial[j * nblk + b] = sum over rows of chunk b of conj(V[:, j]) w
 __global__ void cgemv_c_partial(int n, int k, const cplx* __restrict__ V, long long ldv,
                                 const cplx* __restrict__ w, cplx* __restrict__ partial, int nblk) {
+  join_stream();
   __shared__ double rs[TPB / 32], is[TPB / 32];
   const int b = blockIdx.x, j = blockIdx.y;
   const int r0 = b * DOT_CHUNK, r1 = min(n, r0 + DOT_CHUNK);
@@ -121,6 +122,7 @@ __global__ void cgemv_c_partial(int n, int k, const cplx* __restrict__ V, long l
 }
 
 __global__ void reduce_partials(int k, int nblk, const cplx* __restrict__ partial, cplx* __restrict__ out) {
+  join_stream();
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= k) return;
   cplx s = make_double2(0.0, 0.0);
@@ -130,6 +132,7 @@ __global__ void reduce_partials(int k, int nblk, const cplx* __restrict__ partia
 
 __global__ void cgemv_n_sub_kernel(int n, int k, const cplx* __restrict__ V, long long ldv,
                                    const cplx* __restrict__ h, cplx* __restrict__ w, double sign) {
+  join_stream();
   __shared__ cplx hs[256];
   for (int t = threadIdx.x; t < k; t += blockDim.x) hs[t] = h[t];
   __syncthreads();
@@ -142,6 +145,7 @@ __global__ void cgemv_n_sub_kernel(int n, int k, const cplx* __restrict__ V, lon
 }
 
 __global__ void nrm2_partial(int n, const cplx* __restrict__ x, double* __restrict__ partial) {
+  join_stream();
   __shared__ double rs[TPB / 32];
   const int r0 = blockIdx.x * DOT_CHUNK, r1 = min(n, r0 + DOT_CHUNK);
   double s = 0.0;
@@ -158,6 +162,7 @@ __global__ void nrm2_partial(int n, const cplx* __restrict__ x, double* __restri
 }
 
 __global__ void nrm2_final(int nblk, const double* __restrict__ partial, double* __restrict__ out) {
+  join_stream();
   if (threadIdx.x == 0 && blockIdx.x == 0) {
     double s = 0.0;
     for (int b = 0; b < nblk; b++) s += partial[b];
@@ -167,6 +172,7 @@ __global__ void nrm2_final(int nblk, const double* __restrict__ partial, double*
 
 __global__ void zscal_inv_kernel(int n, const cplx* __restrict__ x, const double* __restrict__ nrm,
                                  cplx* __restrict__ y) {
+  join_stream();
   const double inv = 1.0 / nrm[0];
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x)
@@ -174,18 +180,21 @@ __global__ void zscal_inv_kernel(int n, const cplx* __restrict__ x, const double
 }
 
 __global__ void zaxpby_kernel(int n, cplx a, const cplx* __restrict__ x, cplx b, cplx* __restrict__ y) {
+  join_stream();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x)
     y[i] = cadd(cmul(a, x[i]), cmul(b, y[i]));
 }
 
 __global__ void zcopy_kernel(long long n, const cplx* __restrict__ s, cplx* __restrict__ d) {
+  join_stream();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x)
     d[i] = s[i];
 }
 
 __global__ void zfill_kernel(long long n, cplx v, cplx* __restrict__ d) {
+  join_stream();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x)
     d[i] = v;
@@ -221,6 +230,7 @@ __global__ void site_dev_to_ref_kernel(int d, int Dl, int Dr, const cplx* __rest
 
 __global__ void transpose_pqr_kernel(int P, int Q, int R, const cplx* __restrict__ in,
                                      cplx* __restrict__ out, bool conj) {
+  join_stream();
   const long long n = (long long)P * Q * R;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n;
        t += (long long)gridDim.x * blockDim.x) {
@@ -270,6 +280,7 @@ __device__ __forceinline__ long long view_off(const View2& v, long long i, long 
 
 __global__ void gather2_kernel(int m, int n, const cplx* __restrict__ src, View2 v,
                                cplx* __restrict__ dst) {
+  join_stream();
   const long long tot = (long long)m * n;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < tot;
        t += (long long)gridDim.x * blockDim.x) {
@@ -282,6 +293,7 @@ __global__ void gather2_kernel(int m, int n, const cplx* __restrict__ src, View2
 
 __global__ void scatter2_kernel(int m, int n, const cplx* __restrict__ src, cplx* __restrict__ dst,
                                 View2 v) {
+  join_stream();
   const long long tot = (long long)m * n;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < tot;
        t += (long long)gridDim.x * blockDim.x) {
@@ -319,49 +331,40 @@ void cgemv_c(const Stream& st, int n, int k, const cplx* V, long long ldv, const
   if (k <= 0) return;
   int nblk = ceil_div(n, DOT_CHUNK);
   cplx* partial = (cplx*)scratch.get((size_t)nblk * k * sizeof(cplx));
-  cgemv_c_partial<<<dim3(nblk, k), TPB, 0, st.s>>>(n, k, V, ldv, w, partial, nblk);
-  after_launch(st);
-  reduce_partials<<<ceil_div(k, 64), 64, 0, st.s>>>(k, nblk, partial, dots);
-  after_launch(st);
+  launch_chained(st, cgemv_c_partial, dim3(nblk, k), TPB, 0, n, k, V, ldv, w, partial, nblk);
+  launch_chained(st, reduce_partials, ceil_div(k, 64), 64, 0, k, nblk, partial, dots);
 }
 
 void cgemv_n_sub(const Stream& st, int n, int k, const cplx* V, long long ldv, const cplx* h, cplx* w,
                  double sign) {
   MPSGPU_CHECK(k <= 256, MPSGPU_BAD_SHAPE, "cgemv_n_sub: k > 256");
   if (k <= 0) return;
-  cgemv_n_sub_kernel<<<grid_for(n), TPB, 0, st.s>>>(n, k, V, ldv, h, w, sign);
-  after_launch(st);
+  launch_chained(st, cgemv_n_sub_kernel, grid_for(n), TPB, 0, n, k, V, ldv, h, w, sign);
 }
 
 void dznrm2(const Stream& st, int n, const cplx* x, double* out, Scratch& scratch) {
   int nblk = ceil_div(n, DOT_CHUNK);
   double* partial = (double*)scratch.get((size_t)nblk * sizeof(double));
-  nrm2_partial<<<nblk, TPB, 0, st.s>>>(n, x, partial);
-  after_launch(st);
-  nrm2_final<<<1, 32, 0, st.s>>>(nblk, partial, out);
-  after_launch(st);
+  launch_chained(st, nrm2_partial, nblk, TPB, 0, n, x, partial);
+  launch_chained(st, nrm2_final, 1, 32, 0, nblk, partial, out);
 }
 
 void zscal_inv(const Stream& st, int n, const cplx* x, const double* nrm, cplx* y) {
-  zscal_inv_kernel<<<grid_for(n), TPB, 0, st.s>>>(n, x, nrm, y);
-  after_launch(st);
+  launch_chained(st, zscal_inv_kernel, grid_for(n), TPB, 0, n, x, nrm, y);
 }
 
 void zaxpby(const Stream& st, int n, cplx a, const cplx* x, cplx b, cplx* y) {
-  zaxpby_kernel<<<grid_for(n), TPB, 0, st.s>>>(n, a, x, b, y);
-  after_launch(st);
+  launch_chained(st, zaxpby_kernel, grid_for(n), TPB, 0, n, a, x, b, y);
 }
 
 void zcopy(const Stream& st, int n, const cplx* src, cplx* dst) {
   if (n <= 0) return;
-  zcopy_kernel<<<grid_for(n), TPB, 0, st.s>>>(n, src, dst);
-  after_launch(st);
+  launch_chained(st, zcopy_kernel, grid_for(n), TPB, 0, n, src, dst);
 }
 
 void zfill(const Stream& st, long long n, cplx v, cplx* dst) {
   if (n <= 0) return;
-  zfill_kernel<<<grid_for(n), TPB, 0, st.s>>>(n, v, dst);
-  after_launch(st);
+  launch_chained(st, zfill_kernel, grid_for(n), TPB, 0, n, v, dst);
 }
 
 void site_ref_to_dev(const Stream& st, int d, int Dl, int Dr, const cplx* ref, cplx* dev) {
@@ -375,8 +378,7 @@ void site_dev_to_ref(const Stream& st, int d, int Dl, int Dr, const cplx* dev, c
 }
 
 void transpose_pqr_to_rqp(const Stream& st, int p, int q, int r, const cplx* in, cplx* out, bool conj) {
-  transpose_pqr_kernel<<<grid_for((long long)p * q * r), TPB, 0, st.s>>>(p, q, r, in, out, conj);
-  after_launch(st);
+  launch_chained(st, transpose_pqr_kernel, grid_for((long long)p * q * r), TPB, 0, p, q, r, in, out, conj);
 }
 
 void gaussian_site(const Stream& st, uint64_t seed, long long offset, int d, int Dl, int Dr, cplx* dev) {
@@ -385,13 +387,11 @@ void gaussian_site(const Stream& st, uint64_t seed, long long offset, int d, int
 }
 
 void gather2(const Stream& st, int m, int n, const cplx* src, const View2& v, cplx* dst) {
-  gather2_kernel<<<grid_for((long long)m * n), TPB, 0, st.s>>>(m, n, src, v, dst);
-  after_launch(st);
+  launch_chained(st, gather2_kernel, grid_for((long long)m * n), TPB, 0, m, n, src, v, dst);
 }
 
 void scatter2(const Stream& st, int m, int n, const cplx* src, cplx* dst, const View2& v) {
-  scatter2_kernel<<<grid_for((long long)m * n), TPB, 0, st.s>>>(m, n, src, dst, v);
-  after_launch(st);
+  launch_chained(st, scatter2_kernel, grid_for((long long)m * n), TPB, 0, m, n, src, dst, v);
 }
 
 }  // namespace mpsgpu

@@ -276,6 +276,7 @@ template <class D, class B>
 struct ParamSource {
   using Desc = D;
   struct Slot {};
+  static constexpr bool IN_MEMORY = false;
   static __device__ __forceinline__ const D& pick(const B& b, int t, Slot&) {
     int q = 0;
     while (q + 1 < b.n && b.d[q + 1].tile_begin <= t) q++;
@@ -290,6 +291,7 @@ template <class D>
 struct Source<Extern<D>> {
   using Desc = D;
   using Slot = D;
+  static constexpr bool IN_MEMORY = true;
   static __device__ __forceinline__ const D& pick(const Extern<D>& b, int t, Slot& slot) {
     int lo = 0, hi = b.n - 1;
     while (lo < hi) {
@@ -314,6 +316,7 @@ __global__ void __launch_bounds__(nthreads<BM>(), BM <= 32 ? 3 : 2) heff_gemm1w_
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int NT_ = nthreads<BM>();
   Ring<BM, BN>& ring = *reinterpret_cast<Ring<BM, BN>*>(smem_raw);
+  if (Source<B>::IN_MEMORY) await_predecessor();
   const Gemm1wDesc& d = Source<B>::pick(b, blockIdx.x, slot);
   const int local = blockIdx.x - d.tile_begin;
   const int TX = BM / d.n_i0, TY = BN / d.n_i1;
@@ -328,7 +331,9 @@ __global__ void __launch_bounds__(nthreads<BM>(), BM <= 32 ? 3 : 2) heff_gemm1w_
   Feed<BM, BN> feed;
   feed.start(ring, d.A, d.lda, arow, d.B + (long long)d.n_i1 * y0 * d.ldb, d.ldb, min(TY, d.Y - y0) * d.n_i1);
   Acc<BM, BN, NS> acc;
+  if (!Source<B>::IN_MEMORY) await_predecessor();
   mainloop<BM, BN, NS>(ring, acc, (d.K + BK - 1) / BK, [&](int stage, int slab) { feed.issue(stage, d.K - slab * BK); });
+  admit_successor();
   cplx* Cs = reinterpret_cast<cplx*>(smem_raw);
   constexpr int LD = BN + PADC;
   constexpr int ROOM = (int)(ring_bytes<BM, BN>() - BM * LD * sizeof(cplx));  // behind the tile
@@ -431,6 +436,7 @@ __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(nthreads<BM>(), BM 
   constexpr int NT_ = nthreads<BM>();
   Ring<BM, BN>& ring = *reinterpret_cast<Ring<BM, BN>*>(smem_raw);
   const int tile = blockIdx.x / CS, rank = blockIdx.x % CS;
+  if (Source<B>::IN_MEMORY) await_predecessor();
   const Gemm3Desc& d = Source<B>::pick(b, tile, slot);
   const int local = tile - d.tile_begin;
   const int tm = local % d.tiles_m, tn = local / d.tiles_m;
@@ -451,11 +457,13 @@ __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(nthreads<BM>(), BM 
     feed.skip(s0 - n1);
   }
   Acc<BM, BN, NS> acc;
+  if (!Source<B>::IN_MEMORY) await_predecessor();
   mainloop<BM, BN, NS>(ring, acc, s1 - s0, [&](int stage, int slab) {
     const int sl = s0 + slab;
     if (sl == n1) second();
     feed.issue(stage, sl < n1 ? d.K1 - sl * BK : d.K2 - (sl - n1) * BK);
   });
+  admit_successor();
   cplx* Cs = reinterpret_cast<cplx*>(smem_raw);
   acc_to_smem<BM, BN, NS>(acc, Cs);
   // rows [r0, r1) of the tile are finished by this rank: the sum over the
@@ -548,12 +556,11 @@ template <class B>
 void launch1(const Stream& st, const HeffLaunch& l, const B& b) {
   ProfScope ps(st, GemmProfiler::GEMM64, l.work);
   if (l.bm == 64)
-    heff_gemm1w_kernel<64, 32, 2><<<l.tiles, nthreads<64>(), ring_bytes<64, 32>(), st.s>>>(b);
+    launch_chained(st, heff_gemm1w_kernel<64, 32, 2, B>, l.tiles, nthreads<64>(), ring_bytes<64, 32>(), b);
   else if (l.single)
-    heff_gemm1w_kernel<32, 32, 4><<<l.tiles, nthreads<32>(), ring_bytes<32, 32>(), st.s>>>(b);
+    launch_chained(st, heff_gemm1w_kernel<32, 32, 4, B>, l.tiles, nthreads<32>(), ring_bytes<32, 32>(), b);
   else
-    heff_gemm1w_kernel<32, 32, 2><<<l.tiles, nthreads<32>(), ring_bytes<32, 32>(), st.s>>>(b);
-  after_launch(st);
+    launch_chained(st, heff_gemm1w_kernel<32, 32, 2, B>, l.tiles, nthreads<32>(), ring_bytes<32, 32>(), b);
 }
 
 template <class B>
@@ -561,7 +568,7 @@ void launch3(const Stream& st, const HeffLaunch& l, const B& b) {
   ProfScope ps(st, GemmProfiler::GEMM64, l.work);
   const dim3 grid(l.tiles * l.cs);
 #define MPSGPU_G3(BMv, CSv, NSv) \
-  heff_gemm3_kernel<BMv, 32, CSv, NSv><<<grid, nthreads<BMv>(), ring_bytes<BMv, 32>(), st.s>>>(b)
+  launch_chained(st, heff_gemm3_kernel<BMv, 32, CSv, NSv, B>, grid, nthreads<BMv>(), ring_bytes<BMv, 32>(), b)
   if (l.bm == 64 && l.cs == 1) {
     MPSGPU_G3(64, 1, 2);
   } else if (l.bm == 64 && l.cs == 2) {
@@ -580,7 +587,6 @@ void launch3(const Stream& st, const HeffLaunch& l, const B& b) {
     MPSGPU_G3(32, 8, 2);
   }
 #undef MPSGPU_G3
-  after_launch(st);
 }
 
 // tile ranges and launch shape of a group of first contractions

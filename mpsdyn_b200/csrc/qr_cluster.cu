@@ -625,6 +625,7 @@ __global__ void __launch_bounds__(QT) qr_small_kernel(const __grid_constant__ Qc
   __shared__ cplx C[NB * 33], Ts[NB * T_LD], G[NB * NB], taus[2 * NB], V[2 * MAX_ROWS], W2[NB * W2_LD];
   __shared__ Reflector reflector;
   const int tid = threadIdx.x, m = p.m;
+  join_stream();
   for (int t = tid; t < m * NB; t += QT) {
     const int r = p.a_colfast ? t / NB : t % m, c = p.a_colfast ? t % NB : t / m;
     cplx v = make_double2(0.0, 0.0);
@@ -729,8 +730,7 @@ void cluster_qr(const Stream& st, int m, int n, const cplx* A, const View2& va, 
   // factorisation and explicit Q, complex flops (8 per complex MAC)
   ProfScope ps(st, GemmProfiler::QR, qr_flops(m, n));
   if (m <= 32 && n <= NB) {
-    qr_small_kernel<<<1, QT, 0, st.s>>>(p);
-    after_launch(st);
+    launch_chained(st, qr_small_kernel, 1, QT, 0, p);
     return;
   }
   p.V = (cplx*)scratch.get(((size_t)p.np * m * NB + (size_t)p.np * NB * NB) * sizeof(cplx));

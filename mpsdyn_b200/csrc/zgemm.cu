@@ -198,6 +198,7 @@ __device__ __forceinline__ void tile_store(const double (&acc)[BM / WMW / 8][BN 
 template <int BM, int BN, int WMW, int WNW, int OPA, int OPB>
 __global__ void __launch_bounds__(WMW* WNW * 32)
 zgemm_dmma_kernel(GemmArgs g, int splits, int kchunk, cplx* __restrict__ partial) {
+  join_stream();
   __shared__ TileSmem<BM, BN> sm;
   double acc[BM / WMW / 8][BN / WNW / 8][4][2];
   const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
@@ -217,6 +218,7 @@ zgemm_dmma_kernel(GemmArgs g, int splits, int kchunk, cplx* __restrict__ partial
 }
 
 __global__ void splitk_reduce_kernel(GemmArgs g, int splits, const cplx* __restrict__ partial) {
+  join_stream();
   long long mn = (long long)g.M * g.N;
   long long total = mn * g.batch;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
@@ -238,8 +240,7 @@ void launch_tiles(const Stream& st, const GemmArgs& g, int splits, int kchunk, c
   const int threads = WMW * WNW * 32;
 #define MPSGPU_GEMM_CASE(oa, ob)                                                                    \
   if (g.opA == oa && g.opB == ob) {                                                                 \
-    zgemm_dmma_kernel<BM, BN, WMW, WNW, oa, ob><<<grid, threads, 0, st.s>>>(g, splits, kchunk, partial); \
-    after_launch(st);                                                                               \
+    launch_chained(st, zgemm_dmma_kernel<BM, BN, WMW, WNW, oa, ob>, grid, threads, 0, g, splits, kchunk, partial); \
     return;                                                                                         \
   }
   MPSGPU_GEMM_CASE(OP_N, OP_N)
@@ -285,8 +286,7 @@ void run_cfg(const Stream& st, const GemmArgs& g, GemmCfg c, Scratch& scratch) {
   else launch_tiles<32, 32, 2, 2>(st, g, splits, kchunk, partial);
   if (splits > 1) {
     const long long total = (long long)g.M * g.N * g.batch;
-    splitk_reduce_kernel<<<std::min<long long>(ceil_div(total, 256), 4096), 256, 0, st.s>>>(g, splits, partial);
-    after_launch(st);
+    launch_chained(st, splitk_reduce_kernel, std::min<long long>(ceil_div(total, 256), 4096), 256, 0, g, splits, partial);
   }
 }
 
@@ -399,8 +399,7 @@ void zgemm(const Stream& st, const GemmArgs& g0, Scratch& scratch) {
     GemmArgs z = g;
     z.K = 0;
     long long total = (long long)g.M * g.N * g.batch;
-    splitk_reduce_kernel<<<std::min<long long>(ceil_div(total, 256), 4096), 256, 0, st.s>>>(z, 0, nullptr);
-    after_launch(st);
+    launch_chained(st, splitk_reduce_kernel, std::min<long long>(ceil_div(total, 256), 4096), 256, 0, z, 0, nullptr);
     return;
   }
   const GemmCfg cfg = choose_cfg(st, g, scratch);
