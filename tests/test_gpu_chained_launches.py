@@ -20,8 +20,8 @@ def test_chained_kernels_match_synchronised_ones(ctx, D):
         ctx.synchronize()
     for x, y in zip(a.download()[0], b.download()[0]):
         assert np.array_equal(x, y)
-    one = ctx.contract(a, psi)
+    one = ctx.contract(a, None, psi)
     for _ in range(5):
-        assert ctx.contract(a, psi) == one
+        assert ctx.contract(a, None, psi) == one
     for p in (psi, a, b):
         p.free()
