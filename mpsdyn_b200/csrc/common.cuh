@@ -179,6 +179,19 @@ __device__ __forceinline__ void join_stream() {
   admit_successor();
   await_predecessor();
 }
+
+// Of n ascending first elements begin(q), the last that is not above t; the same t
+// in every thread of the block, which all take part: one round of loads instead of
+// a chain of them.
+template <class F>
+__device__ __forceinline__ int block_find(int n, long long t, F begin) {
+  int c = 0;
+  for (int q0 = 0; q0 < n; q0 += blockDim.x) {
+    const int q = q0 + threadIdx.x;
+    c += __syncthreads_count(q < n && begin(q) <= t);
+  }
+  return c > 0 ? c - 1 : 0;
+}
 #endif
 
 inline int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }

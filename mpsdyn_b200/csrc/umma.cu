@@ -408,23 +408,21 @@ __global__ void split_reduce_kernel(int M, int N, int splits, const cplx* __rest
 // job j (t in [begin_j, begin_{j+1})) is C[m + n ldc] = alpha sum_s part[s M N
 // + m + n M] + beta Cin[m + n ldcin], the partials added in order.
 __global__ void split_reduce_grouped_kernel(const SplitReduceJob* __restrict__ jobs, int n, long long total) {
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
-       t += (long long)gridDim.x * blockDim.x) {
-    int lo = 0, hi = n - 1;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (jobs[mid].begin <= t) lo = mid;
-      else hi = mid - 1;
-    }
+  for (long long t0 = (long long)blockIdx.x * blockDim.x; t0 < total; t0 += (long long)gridDim.x * blockDim.x) {
+    int lo = block_find(n, t0, [&](int q) { return jobs[q].begin; });
+    const long long t = t0 + threadIdx.x;
+    if (t >= total) continue;
+    while (lo + 1 < n && jobs[lo + 1].begin <= t) lo++;
     const SplitReduceJob& jb = jobs[lo];
     const long long e = t - jb.begin, mn = (long long)jb.M * jb.N;
-    const int m = (int)(e % jb.M);
-    const long long col = e / jb.M;
+    const int col = mn <= 0x7fffffff ? (int)e / jb.M : (int)(e / jb.M);
+    const int m = (int)(e - (long long)col * jb.M);
     cplx s = cmake(0.0, 0.0);
+#pragma unroll 4
     for (int p = 0; p < jb.nparts; p++) s = cadd(s, jb.part[p * mn + e]);
     cplx o = cmul(jb.alpha, s);
-    if (jb.Cin) o = cadd(o, cmul(jb.beta, jb.Cin[m + col * jb.ldcin]));
-    jb.C[m + col * jb.ldc] = o;
+    if (jb.Cin) o = cadd(o, cmul(jb.beta, jb.Cin[m + (long long)col * jb.ldcin]));
+    jb.C[m + (long long)col * jb.ldc] = o;
   }
 }
 
@@ -446,45 +444,37 @@ void launch_split(const Stream& st, const SplitGemmParams& p, const SplitGroupPa
   after_launch(st);
 }
 
-// Grouped operand preparation: job j covers threads [thread_begin, next);
-// every operand is tiled with 128-row tiles.
-__global__ void split_prepare_grouped_kernel(const SplitPrepJob* __restrict__ jobs, int n, long long total) {
+// Grouped operand preparation: job j covers threads [thread_begin, next); every
+// operand is tiled with 128-row tiles, so a block of 256 threads prepares one
+// (row tile, k-step).
+constexpr int PREP_THREADS = 2 * SP_BM;
+__global__ void __launch_bounds__(PREP_THREADS) split_prepare_grouped_kernel(const SplitPrepJob* __restrict__ jobs, int n,
+                                                                             long long total) {
   constexpr int RT = SP_BM;
-  constexpr int groups = RT / 8;
   constexpr int plane = sp_plane_bytes(RT);
-  for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-       idx += (long long)gridDim.x * blockDim.x) {
-    int lo = 0, hi = n - 1;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (jobs[mid].thread_begin <= idx) lo = mid;
-      else hi = mid - 1;
-    }
-    const SplitPrepJob& jb = jobs[lo];
-    const long long li = idx - jb.thread_begin;
-    const int r = (int)(li & 7);
-    long long q = li >> 3;
-    const int g = (int)(q % groups);
-    q /= groups;
-    const int kg = (int)(q & 1);
-    q >>= 1;
-    const int ks = (int)(q % jb.KS);
-    const long long rt = q / jb.KS;
-    const long long row = rt * RT + g * 8 + r;
+  const int r = threadIdx.x & 7, g = (threadIdx.x >> 3) % (RT / 8), kg = threadIdx.x / RT;
+  for (long long t0 = (long long)blockIdx.x * PREP_THREADS; t0 < total; t0 += (long long)gridDim.x * PREP_THREADS) {
+    const SplitPrepJob& jb = jobs[block_find(n, t0, [&](int q) { return jobs[q].thread_begin; })];
+    const unsigned tile = (unsigned)((t0 - jb.thread_begin) / PREP_THREADS);
+    const int rt = tile / jb.KS, ks = tile % jb.KS;
+    const long long row = (long long)rt * RT + g * 8 + r;
     const int k0 = ks * SP_BK + kg * 8;
     union {
       __nv_bfloat16 h[8];
       uint4 u;
     } pk[SP_PLANES];
+    cplx x[8];
 #pragma unroll
     for (int kk = 0; kk < 8; kk++) {
       const int k = k0 + kk;
-      cplx x = cmake(0.0, 0.0);
-      if (row < jb.rows && k < jb.K) x = jb.X[row * jb.rs + (long long)k * jb.ks];
-      split3(x.x, pk[0].h[kk], pk[1].h[kk], pk[2].h[kk]);
-      split3(x.y, pk[3].h[kk], pk[4].h[kk], pk[5].h[kk]);
+      x[kk] = row < jb.rows && k < jb.K ? jb.X[row * jb.rs + (long long)k * jb.ks] : cmake(0.0, 0.0);
     }
-    uint8_t* base = jb.out + ((rt * jb.KS + ks) * SP_PLANES) * plane + (long long)kg * (RT * 16) + g * 128 + r * 16;
+#pragma unroll
+    for (int kk = 0; kk < 8; kk++) {
+      split3(x[kk].x, pk[0].h[kk], pk[1].h[kk], pk[2].h[kk]);
+      split3(x[kk].y, pk[3].h[kk], pk[4].h[kk], pk[5].h[kk]);
+    }
+    uint8_t* base = jb.out + (((long long)rt * jb.KS + ks) * SP_PLANES) * plane + kg * (RT * 16) + g * 128 + r * 16;
 #pragma unroll
     for (int p = 0; p < SP_PLANES; p++) *reinterpret_cast<uint4*>(base + (long long)p * plane) = pk[p].u;
   }
@@ -616,8 +606,8 @@ long long split_prepare_jobs(SplitPrepJob* jobs, int n) {
 }
 
 void split_prepare_grouped(const Stream& st, const SplitPrepJob* d_jobs, int n, long long threads) {
-  const int blocks = (int)std::min<long long>((threads + 255) / 256, 148LL * 16);
-  split_prepare_grouped_kernel<<<blocks, 256, 0, st.s>>>(d_jobs, n, threads);
+  const int blocks = (int)std::min<long long>((threads + PREP_THREADS - 1) / PREP_THREADS, 148LL * 16);
+  split_prepare_grouped_kernel<<<blocks, PREP_THREADS, 0, st.s>>>(d_jobs, n, threads);
   after_launch(st);
 }
 
