@@ -130,16 +130,17 @@ double grouped_matvec_flops(const HeffInstance& h) {
 void grouped_matvec_plan(const Stream& st, const std::vector<HeffInstance>& inst, GroupedMatvecPlan& plan) {
   const int n = (int)inst.size();
   const std::vector<int> order = grouped_matvec_order(inst);
-  long long t1_total = 0, wm_total = 0, pix_total = 0, wel_total = 0;
+  long long t1_total = 0, t2_total = 0, wm_total = 0, pix_total = 0, wel_total = 0;
   for (const auto& h : inst) {
     t1_total += (long long)h.Dl * h.wl * h.d * h.Dr;
+    t2_total += (long long)h.Dl * h.d * h.wr * h.Dr;
     wm_total += (long long)h.d * h.wl * h.d * h.wr;
     pix_total += (long long)h.Dl * h.Dr;
   }
   wel_total = wm_total;
   plan.n = n;
   dbuf_alloc(st, plan.t1, t1_total);
-  dbuf_alloc(st, plan.t2, t1_total);
+  dbuf_alloc(st, plan.t2, t2_total);
   dbuf_alloc(st, plan.wm, wm_total);
   std::vector<WGroup> wg(n);
   std::vector<WPerm> wp(n);
@@ -153,14 +154,14 @@ void grouped_matvec_plan(const Stream& st, const std::vector<HeffInstance>& inst
     spb += (bytes + 255) / 256 * 256;
     return o;
   };
-  long long o1 = 0, ow = 0, pix = 0;
+  long long o1 = 0, o2 = 0, ow = 0, pix = 0;
   int maxnin = 1, maxnout = 1;
   for (int q = 0; q < n; q++) {
     const int i = order[q];
     const HeffInstance& h = inst[i];
     const int d = h.d, wl = h.wl, wr = h.wr, Dl = h.Dl, Dr = h.Dr;
     cplx* T1 = plan.t1.p + o1;
-    cplx* T2 = plan.t2.p + o1;
+    cplx* T2 = plan.t2.p + o2;
     cplx* Wm = plan.wm.p + ow;
     wp[q] = WPerm{h.W, Wm, d, wl, d, wr, ow};
     WContractArgs& w = wg[q].a;
@@ -172,6 +173,7 @@ void grouped_matvec_plan(const Stream& st, const std::vector<HeffInstance>& inst
     w.Wm = Wm;
     wg[q].pix_begin = pix;
     o1 += (long long)Dl * wl * d * Dr;
+    o2 += (long long)Dl * d * wr * Dr;
     ow += (long long)d * wl * d * wr;
     pix += wcontract_chunked((long long)Dl * Dr);
     maxnin = std::max(maxnin, wl * d);
