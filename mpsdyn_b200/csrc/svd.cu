@@ -127,11 +127,16 @@ __device__ __forceinline__ bool jacobi_pair(cplx* ap, cplx* aq, int m, cplx* vp,
       return true;
     }
   }
-  const double g = sqrt(cabs2(ga));
-  if (!(g > JTOL * sqrt(al * be) && g > 1e-300)) return false;
+  const double g = sqrt(cabs2(ga)), ab = al * be;
+  // (the product underflows for two columns of 1e-80, each square does not)
+  if (!(g > JTOL * (ab > 1e-280 ? sqrt(ab) : sqrt(al) * sqrt(be)) && g > 1e-300)) return false;
   // rotate (a_p, a_q conj(phase)) so that the pair becomes orthogonal
   const double zeta = (be - al) / (2.0 * g);
   const double t = (zeta >= 0 ? 1.0 : -1.0) / (fabs(zeta) + sqrt(1.0 + zeta * zeta));
+  // no rotation (zeta^2 overflows: the smaller column is below 1e-154 of the
+  // larger, as what is left of parallel columns gets after some sweeps); counted
+  // as one it kept the sweeps from ending
+  if (t == 0.0) return false;
   const double cs = 1.0 / sqrt(1.0 + t * t), sn = cs * t;
   const cplx ph = make_double2(ga.x / g, -ga.y / g);  // conj(gamma)/|gamma|
   rotate_phase(ap, aq, m, cs, sn, ph);

@@ -75,3 +75,29 @@ def test_cuts_match_lapack(ctx, d, L, D, cut):
     assert abs(discarded - dropped) < 1e-12 * max(dropped, abs(wnorm) ** 2)
     assert abs(abs(overlap(got, want)) - 1) < 1e-11
     assert abs(overlap(got, got) - 1) < 1e-11
+
+
+@pytest.mark.parametrize("D", [2, 7, 16, 24, 40])
+def test_parallel_columns_settle(ctx, D):
+    """Columns parallel to the first one shrink by a rounding error a sweep, to zero through values whose squares
+    underflow: the last site's matrix of rank 1 with columns of falling size, cut to all of them."""
+    rs = np.random.RandomState(D)
+    d = max(2, D)
+    A = rs.standard_normal((d, 1, D)) + 1j * rs.standard_normal((d, 1, D))
+    B = np.zeros((d, D, 1), dtype=complex)
+    B[0, :, 0] = rs.standard_normal(D) * 10.0 ** -np.linspace(0, 17, D)
+    cut, disc = ctx.mps([np.asfortranarray(A), np.asfortranarray(B)]).approximate(D)
+    assert abs(np.max(ctx.schmidt_values(cut, 1)) - 1.0) < 1e-12 and disc < 1e-24
+
+
+@pytest.mark.parametrize("D", [12, 24, 40])
+def test_doubly_graded_matrix_settles(ctx, D):
+    """Rows and columns that both fall off by 1e-3 an index: pairs of columns of 1e-80, whose squares' product
+    underflows."""
+    rs = np.random.RandomState(D)
+    g = 10.0 ** -(np.arange(D) * 100.0 / D)
+    M = g[:, None] * (rs.standard_normal((D, D)) + 1j * rs.standard_normal((D, D))) * g
+    A = rs.standard_normal((D, 1, D)) + 1j * rs.standard_normal((D, 1, D))
+    cut, disc = ctx.mps([np.asfortranarray(A), np.asfortranarray(M.reshape(D, D, 1))]).approximate(D)
+    s = np.linalg.svd(A[:, 0] @ M.T, compute_uv=False)
+    assert abs(np.max(ctx.schmidt_values(cut, 1)) - s[0] ** 2 / np.sum(s**2)) < 1e-12 and disc < 1e-24
