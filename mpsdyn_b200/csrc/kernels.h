@@ -353,6 +353,8 @@ void zaxpby(const Stream& st, int n, cplx a, const cplx* x, cplx b, cplx* y);
 // dst = src (n complex)
 void zcopy(const Stream& st, int n, const cplx* src, cplx* dst);
 void zfill(const Stream& st, long long n, cplx v, cplx* dst);
+// entries with both parts below tiny become zero
+void zflush(const Stream& st, long long n, double tiny, cplx* x);
 
 // ---- layout conversions between the reference and the device layout ----
 // site: ref A(s, a, r) -> dev X(a, s, r) and back
