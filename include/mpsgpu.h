@@ -431,7 +431,7 @@ mpsgpu_status mpsgpu_heff_matvec(mpsgpu_context* ctx, const int* ldims,
  *   W  (d, wl, d, wr) MPO tensor, as the reference stores it
  *   Rt (Dr, wr, Dr)  right environment in (ket, w, bra) order
  *   x, y (Dl, d, Dr) site vector with the left bond fastest
- * The three grouped launches (GEMM, MPO-leg contraction, GEMM) run once; with
+ * The grouped launches (two in FP64: L.x with the MPO legs, and .Rt) run once; with
  * repeats > 0 they are captured in a CUDA graph and replayed `repeats` times,
  * and *ms_per_run gets the device time per product (CUDA events).  *flops
  * gets the algorithmic flops of one grouped product. */
