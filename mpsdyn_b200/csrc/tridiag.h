@@ -1,9 +1,9 @@
 // Lowest eigenpair of a real symmetric tridiagonal matrix (the projected
 // Rayleigh-Ritz problem of the Lanczos iteration, kept in FP64 on the host:
-// k <= 256, O(k) per bisection step).
+// k <= 256, O(k) per step).
 //
-// Eigenvalue: bisection on the Gershgorin interval with Sturm-sequence
-// counts (the number of negative pivots of the LDL^T factorisation of
+// Eigenvalue: Newton's iteration from below (solve_from), or bisection on the
+// Gershgorin interval with Sturm-sequence counts (the number of negative pivots of the LDL^T factorisation of
 // T - x I equals the number of eigenvalues below x; Wilkinson, "The
 // Algebraic Eigenvalue Problem", 5.38).  Eigenvector: inverse iteration
 // on T - theta I with a row-pivoted tridiagonal elimination.
