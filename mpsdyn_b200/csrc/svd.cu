@@ -20,8 +20,9 @@
 // (Contractor::getSchmidtValues / getEntropy, Contractor.cpp:2045-2076 and
 // :2243-2270: there the eigenvalues of the reduced density matrix; here the
 // squares of the singular values of the bond matrix, which are the same
-// numbers and carry full relative accuracy for the small ones), and for the cut
-// SVDs of MPO application and two-site sweeps.
+// numbers and carry full relative accuracy for the small ones, as long as the
+// products of two columns stay above 1e-154), and for the cut SVDs of MPO
+// application and two-site sweeps.
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -127,9 +128,13 @@ __device__ __forceinline__ bool jacobi_pair(cplx* ap, cplx* aq, int m, cplx* vp,
       return true;
     }
   }
-  const double g = sqrt(cabs2(ga)), ab = al * be;
-  // (the product underflows for two columns of 1e-80, each square does not)
-  if (!(g > JTOL * (ab > 1e-280 ? sqrt(ab) : sqrt(al) * sqrt(be)) && g > 1e-300)) return false;
+  const double g2 = cabs2(ga), g = sqrt(g2), ab = al * be;
+  // Products whose square is below the normal range are left alone: their root,
+  // and with it the modulus of the phase below, is off by up to 40 %, and the
+  // column it multiplies may be a large one (a second value of 1.7e-6 beside
+  // columns of 1e-150 came out 20 % off).
+  // (ab underflows for two columns of 1e-80, each square does not)
+  if (!(g2 >= 2.3e-308 && g > JTOL * (ab > 1e-280 ? sqrt(ab) : sqrt(al) * sqrt(be)))) return false;
   // rotate (a_p, a_q conj(phase)) so that the pair becomes orthogonal
   const double zeta = (be - al) / (2.0 * g);
   const double t = (zeta >= 0 ? 1.0 : -1.0) / (fabs(zeta) + sqrt(1.0 + zeta * zeta));

@@ -101,3 +101,22 @@ def test_doubly_graded_matrix_settles(ctx, D):
     cut, disc = ctx.mps([np.asfortranarray(A), np.asfortranarray(M.reshape(D, D, 1))]).approximate(D)
     s = np.linalg.svd(A[:, 0] @ M.T, compute_uv=False)
     assert abs(np.max(ctx.schmidt_values(cut, 1)) - s[0] ** 2 / np.sum(s**2)) < 1e-12 and disc < 1e-24
+
+
+@pytest.mark.parametrize("low", [1e-150, 1e-155, 1e-160])
+@pytest.mark.parametrize("D", [12, 20, 40, 300])
+def test_tiny_columns_leave_the_large_ones_alone(ctx, D, low):
+    """A matrix whose first two rows hold its two largest values and the others are of `low`, where squares of products
+    underflow: the weight that a cut to one value discards is the second value's square, |det| / s_1 of the first two rows."""
+    rs = np.random.RandomState(D)
+    G = rs.standard_normal((D, D)) + 1j * rs.standard_normal((D, D))
+    c = np.full(D, low) * 10.0 ** rs.uniform(-5, 5, D)
+    c[:2] = 1.0, 1.7e-6
+    U = np.linalg.qr(rs.standard_normal((D, D)) + 1j * rs.standard_normal((D, D)))[0]
+    psi = ctx.mps([np.asfortranarray(U.reshape(D, 1, D)), np.asfortranarray((c[:, None] * G).reshape(D, D, 1))])
+    phi, discarded = psi.approximate(1)
+    psi.free()
+    phi.free()
+    R = np.linalg.qr(G[:2].conj().T)[1]
+    s1 = np.linalg.norm(c[:2, None] * R.conj().T, 2)
+    assert abs(discarded / (c[1] * abs(R[0, 0] * R[1, 1]) / s1) ** 2 - 1.0) < 1e-12
