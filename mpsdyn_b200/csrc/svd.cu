@@ -21,7 +21,7 @@
 // :2243-2270: there the eigenvalues of the reduced density matrix; here the
 // squares of the singular values of the bond matrix, which are the same
 // numbers and carry full relative accuracy for the small ones, as long as the
-// products of two columns stay above 1e-154), and for the cut SVDs of MPO
+// products of two columns stay above 1e-162), and for the cut SVDs of MPO
 // application and two-site sweeps.
 #include <cooperative_groups.h>
 
@@ -128,13 +128,22 @@ __device__ __forceinline__ bool jacobi_pair(cplx* ap, cplx* aq, int m, cplx* vp,
       return true;
     }
   }
-  const double g2 = cabs2(ga), g = sqrt(g2), ab = al * be;
-  // Products whose square is below the normal range are left alone: their root,
-  // and with it the modulus of the phase below, is off by up to 40 %, and the
-  // column it multiplies may be a large one (a second value of 1.7e-6 beside
-  // columns of 1e-150 came out 20 % off).
+  const double g2 = cabs2(ga), ab = al * be;
+  double g = sqrt(g2);
+  if (g2 < 2.3e-308) {
+    // |gamma| from its larger part: the root of a square below the normal range,
+    // and with it the modulus of the phase below, is off by up to 40 %, and the
+    // column it multiplies may be a large one (a second value of 1.7e-6 beside
+    // columns of 1e-150 came out 20 % off).  Where the square vanishes the pair is
+    // left alone: settling values below 1e-81 can
+    // take more than the 40 sweeps (44 at 300 columns graded over ten decades).
+    const double mx = fmax(fabs(ga.x), fabs(ga.y));
+    if (!(mx >= 2.3e-162)) return false;
+    const double x = ga.x / mx, y = ga.y / mx;
+    g = mx * sqrt(fma(x, x, y * y));
+  }
   // (ab underflows for two columns of 1e-80, each square does not)
-  if (!(g2 >= 2.3e-308 && g > JTOL * (ab > 1e-280 ? sqrt(ab) : sqrt(al) * sqrt(be)))) return false;
+  if (!(g > JTOL * (ab > 1e-280 ? sqrt(ab) : sqrt(al) * sqrt(be)))) return false;
   // rotate (a_p, a_q conj(phase)) so that the pair becomes orthogonal
   const double zeta = (be - al) / (2.0 * g);
   const double t = (zeta >= 0 ? 1.0 : -1.0) / (fabs(zeta) + sqrt(1.0 + zeta * zeta));

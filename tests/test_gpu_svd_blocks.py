@@ -120,3 +120,20 @@ def test_tiny_columns_leave_the_large_ones_alone(ctx, D, low):
     R = np.linalg.qr(G[:2].conj().T)[1]
     s1 = np.linalg.norm(c[:2, None] * R.conj().T, 2)
     assert abs(discarded / (c[1] * abs(R[0, 0] * R[1, 1]) / s1) ** 2 - 1.0) < 1e-12
+
+
+@pytest.mark.parametrize("scale", [1e-76, 1e-77])
+@pytest.mark.parametrize("D", [12, 20, 40, 300])
+def test_values_of_tiny_matrices(ctx, D, scale):
+    """A matrix whose columns are all so small that squares of their products underflow: a cut discards the same share
+    of the weight as at scale one (pairs left alone, with products below 2e-162, are orthogonal to 1e-8 there)."""
+    rs = np.random.RandomState(D)
+    cut = min(D // 2, 20)
+    G = rs.standard_normal((D, D)) + 1j * rs.standard_normal((D, D))
+    U = np.linalg.qr(rs.standard_normal((D, D)) + 1j * rs.standard_normal((D, D)))[0]
+    psi = ctx.mps([np.asfortranarray(U.reshape(D, 1, D)), np.asfortranarray((scale * G).reshape(D, D, 1))])
+    phi, discarded = psi.approximate(cut)
+    psi.free()
+    phi.free()
+    s = np.linalg.svd(G, compute_uv=False)
+    assert abs(discarded / scale / scale / np.sum(s[cut:] ** 2) - 1.0) < 1e-12
