@@ -202,13 +202,6 @@ __global__ void zfill_kernel(long long n, cplx v, cplx* __restrict__ d) {
 
 // ---- layouts -----------------------------------------------------------------
 // ref A(s, a, r) at s + d a + d Dl r  <->  dev X(a, s, r) at a + Dl s + Dl d r
-__global__ void zflush_kernel(long long n, double tiny, cplx* __restrict__ x) {
-  join_stream();
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x)
-    if (fabs(x[i].x) < tiny && fabs(x[i].y) < tiny) x[i] = make_double2(0.0, 0.0);
-}
-
 __global__ void site_ref_to_dev_kernel(int d, int Dl, int Dr, const cplx* __restrict__ ref,
                                        cplx* __restrict__ dev) {
   const long long n = (long long)d * Dl * Dr;
@@ -372,11 +365,6 @@ void zcopy(const Stream& st, int n, const cplx* src, cplx* dst) {
 void zfill(const Stream& st, long long n, cplx v, cplx* dst) {
   if (n <= 0) return;
   launch_chained(st, zfill_kernel, grid_for(n), TPB, 0, n, v, dst);
-}
-
-void zflush(const Stream& st, long long n, double tiny, cplx* x) {
-  if (n <= 0) return;
-  launch_chained(st, zflush_kernel, grid_for(n), TPB, 0, n, tiny, x);
 }
 
 void site_ref_to_dev(const Stream& st, int d, int Dl, int Dr, const cplx* ref, cplx* dev) {

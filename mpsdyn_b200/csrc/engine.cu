@@ -2990,7 +2990,7 @@ void expectation_local(Context& c, const MpsDev& s, const double* op, double* ou
 // chain and back does three times as many factorisations one after another.
 // Returns false, for the sweep to decide, where the product could lose accuracy
 // or range: factors whose norms lie near the limits of the type, or a
-// product far below theirs, as of a zero state.
+// product far below theirs, as of a zero state; and where its rotations do not settle.
 static bool schmidt_two_chains(Context& c, const MpsDev& s, int pos, std::vector<double>& sv) {
   const int L = s.L;
   MpsDev aux;
@@ -3000,6 +3000,7 @@ static bool schmidt_two_chains(Context& c, const MpsDev& s, int pos, std::vector
     int kl = 0, kr = 0;
     const int D = s.dims[pos][1];
     double nrm[2];
+    std::vector<cplx> diag[2];  // of the factors
     {
       SecondStream two(c);
       Context& o = two.sub;
@@ -3021,8 +3022,19 @@ static bool schmidt_two_chains(Context& c, const MpsDev& s, int pos, std::vector
       two.join();
       MPSGPU_CUDA(cudaMemcpyAsync(&nrm[0], c.dscal, sizeof(double), cudaMemcpyDeviceToHost, c.stream));
       MPSGPU_CUDA(cudaMemcpyAsync(&nrm[1], o.dscal, sizeof(double), cudaMemcpyDeviceToHost, c.stream));
+      for (int i = 0; i < 2; i++) {
+        const int k = i ? kr : kl;
+        diag[i].resize(std::min(k, D));
+        MPSGPU_CUDA(cudaMemcpy2DAsync(diag[i].data(), sizeof(cplx), i ? o.matR.p : c.matR.p, (k + 1) * sizeof(cplx),
+                                      sizeof(cplx), diag[i].size(), cudaMemcpyDeviceToHost, c.stream));
+      }
       MPSGPU_CUDA(cudaStreamSynchronize(c.stream));
     }
+    auto least = [&](int i) {
+      double v = HUGE_VAL;
+      for (const cplx& z : diag[i]) v = std::min(v, std::fabs(z.x) + std::fabs(z.y));
+      return v / nrm[i];
+    };
     bool ok = true;
     for (double v : nrm) ok = ok && v > 1e-140 && v < 1e140;  // (false for NaN)
     if (ok) {
@@ -3034,16 +3046,20 @@ static bool schmidt_two_chains(Context& c, const MpsDev& s, int pos, std::vector
       g.C = c.t3.p; g.ldc = kl;
       g.alpha = make_double2(1.0 / nrm[0] / nrm[1], 0.0);
       zgemm(c.st(), g, c.scratch);
-      // where the bonds are larger than the rank, the factors' rows fall off by a
-      // rounding error per site (1e-17, 1e-34, ...) and the rotations would take
-      // twice the sweeps to settle them; entries that small are far below the
-      // rounding of the values
-      zflush(c.st(), (long long)kl * kr, 1e-22, c.t3.p);
-      got = singular_values(c.st(), kl, kr, c.t3.p, kl, c.scratch);
+      // No entry is too small to keep: the product holds values that fall off over
+      // many orders to a few ulps each.  Rotations settle in few sweeps when they
+      // work on the side that falls off further (a quench at D = 64: 9 sweeps on
+      // the rows, 43 on the columns); one that takes too many is left to the sweep.
+      try {
+        got = singular_values(c.st(), kl, kr, c.t3.p, kl, c.scratch, least(0) < least(1));
+      } catch (const Error& e) {
+        if (e.status != MPSGPU_NOT_CONVERGED) throw;
+        ok = false;
+      }
       double sum = 0.0;
       for (double v : got) sum += v * v;
       // a canonical half has singular values 1 (norm sqrt(k)); the product then has 1 / sqrt(k)
-      ok = sum * got.size() * got.size() >= 1e-2;
+      ok = ok && sum * got.size() * got.size() >= 1e-2;
       const double n = std::sqrt(sum);
       for (double& v : got) v /= n;
     }

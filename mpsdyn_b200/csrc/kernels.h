@@ -353,8 +353,6 @@ void zaxpby(const Stream& st, int n, cplx a, const cplx* x, cplx b, cplx* y);
 // dst = src (n complex)
 void zcopy(const Stream& st, int n, const cplx* src, cplx* dst);
 void zfill(const Stream& st, long long n, cplx v, cplx* dst);
-// entries with both parts below tiny become zero
-void zflush(const Stream& st, long long n, double tiny, cplx* x);
 
 // ---- layout conversions between the reference and the device layout ----
 // site: ref A(s, a, r) -> dev X(a, s, r) and back
@@ -371,9 +369,10 @@ void gaussian_site(const Stream& st, uint64_t seed, long long offset, int d, int
                    cplx* dev);
 
 // Singular values (descending) of the m x n matrix A (device, ld lda) by
-// one-sided Jacobi (svd.cu); host-synchronous, A untouched.
+// one-sided Jacobi (svd.cu), rotating the shorter side, of a square matrix the
+// columns or (`rows`) the rows; host-synchronous, A untouched.
 std::vector<double> singular_values(const Stream& st, int m, int n, const cplx* A, long long lda,
-                                    Scratch& scratch);
+                                    Scratch& scratch, bool rows = false);
 // Thin SVD with the cut of wrapper::svd(A, 0, cut): U (m x keep, ld m),
 // diag(s) V^H (keep x n, ld keep); all min(m, n) values in sv; returns keep.
 int svd_cut(const Stream& st, int m, int n, const cplx* A, long long lda, int cut, cplx* U, cplx* SVh,

@@ -381,10 +381,10 @@ void jacobi_launch(const Stream& st, int rows, int colsp, cplx* W, cplx* V, doub
 // Singular values (descending) of the m x n matrix at A (device, ld m);
 // A is not modified.  Host-synchronous (returns the values on the host).
 std::vector<double> singular_values(const Stream& st, int m, int n, const cplx* A, long long lda,
-                                    Scratch& scratch) {
+                                    Scratch& scratch, bool by_rows) {
   MPSGPU_CHECK(m > 0 && n > 0, MPSGPU_BAD_SHAPE, "singular_values: empty matrix");
   // work on the orientation with at most as many columns as rows
-  const bool tr = n > m;
+  const bool tr = n > m || (by_rows && n == m);
   const int rows = tr ? n : m;
   int cols = tr ? m : n;
   const int colsp = jacobi_cols(cols);  // zero columns added

@@ -105,3 +105,48 @@ def test_local_observables_of_every_site(ctx, L, d, bonds):
     for k in range(L):
         w = np.moveaxis(np.tensordot(op, v, axes=(1, k)), 0, k)
         assert abs(got[k] - (np.vdot(v, w) / np.vdot(v, v)).real) < TOL
+
+
+@pytest.mark.parametrize("split", [False, True])
+@pytest.mark.parametrize("D", [12, 20, 40])
+def test_graded_schmidt_values(ctx, D, split):
+    """Coefficients that fall evenly from 1 to 1e-40, on one site or split over both: every one to a few ulps of itself
+    (a factorisation, a product and the rotations keep the columns' scales)."""
+    rs = np.random.RandomState(D)
+    U, V = (np.linalg.qr(rs.standard_normal((D, D)) + 1j * rs.standard_normal((D, D)))[0] for _ in range(2))
+    s = 10.0 ** -np.linspace(0, 40, D)
+    left, right = (np.sqrt(s), np.sqrt(s)) if split else (np.ones(D), s)
+    psi = ctx.mps([np.asfortranarray((U * left).reshape(D, 1, D)), np.asfortranarray((right[:, None] * V).T.reshape(D, D, 1))])
+    got = np.sort(ctx.schmidt_values(psi, 1))
+    psi.free()
+    want = np.sort(s**2 / np.sum(s**2))
+    assert np.max(np.abs(got / want - 1.0)) < TOL
+
+
+@pytest.mark.parametrize("flip", [False, True])
+@pytest.mark.parametrize("D", [24, 64])
+def test_schmidt_values_after_a_quench(ctx, D, flip):
+    """Short evolution from a product state at bonds far above its rank: factors whose rows fall off by tens of orders,
+    further on one side of the bond than on the other; every bond of the chain and of its mirror image settles, with the
+    Schmidt values of the two halves' Gram matrices."""
+    L = 24
+    U = ctx.mpo_ising_evolution(L, 1.0, 1.3, 0.1, 0.01, False)
+    psi, o = ctx.mps_product(L, 2, 1), ctx.options(convtol=1e-10)
+    for _ in range(8):
+        aux = psi.copy()
+        ctx.optimize(U, aux, psi, D, o)
+        aux.free()
+    sites = psi.download()[0]
+    if flip:
+        sites = [np.asfortranarray(np.transpose(A, (0, 2, 1))) for A in sites[::-1]]
+    state = ctx.mps(sites)
+    for pos in range(1, L):
+        G, H = np.ones((1, 1)), np.ones((1, 1))
+        for A in sites[:pos]:
+            G = np.einsum("ab,sar,sbt->rt", G, A.conj(), A, optimize=True)
+        for A in sites[pos:][::-1]:
+            H = np.einsum("ab,sra,stb->rt", H, A, A.conj(), optimize=True)
+        lam = np.sort(np.linalg.eigvals(G @ H).real)[::-1]
+        check_schmidt(ctx.schmidt_values(state, pos), lam / lam.sum(), 4 * TOL)
+    for x in (U, psi, state):
+        x.free()
