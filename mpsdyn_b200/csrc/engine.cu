@@ -3118,20 +3118,14 @@ void schmidt_values(Context& c, const MpsDev& s, int pos, std::vector<double>& v
 }
 
 // Contractor::getEntropy (Contractor.cpp:2045-2076): -sum lambda log2 lambda
-// over |lambda| > 1e-12.  The values add up to 1, so the logarithm of one above a
-// half is taken from the sum of the others: rounded next to 1, a value holds no more
-// than three digits of an entropy of 1e-13, whichever way it was computed.
+// over |lambda| > 1e-12.
 double entropy(Context& c, const MpsDev& s, int pos) {
   if (pos == s.L) return 0.0;
-  std::vector<double> lam;  // ascending
+  std::vector<double> lam;
   schmidt_values(c, s, pos, lam);
-  double S = 0.0, rest = 0.0;
-  for (size_t i = 0; i < lam.size(); i++) {
-    const double t = lam[i];
-    const bool tail = i + 1 == lam.size() && rest < 0.5;
-    if (std::fabs(t) > 1e-12) S -= t * (tail ? std::log1p(-rest) / std::log(2.0) : std::log2(t));
-    rest += t;
-  }
+  double S = 0.0;
+  for (double t : lam)
+    if (std::fabs(t) > 1e-12) S += -t * std::log2(t);
   return S;
 }
 

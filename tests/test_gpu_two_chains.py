@@ -150,21 +150,3 @@ def test_schmidt_values_after_a_quench(ctx, D, flip):
         check_schmidt(ctx.schmidt_values(state, pos), lam / lam.sum(), 4 * TOL)
     for x in (U, psi, state):
         x.free()
-
-
-@pytest.mark.parametrize("D", [2, 16, 17, 40])
-@pytest.mark.parametrize("small", [3e-7, 1e-5, 0.3])
-def test_entropy_of_nearly_product_states(ctx, D, small):
-    """Two coefficients, cos and sin of an angle, in a bond of D: entropies of 1e-13 and 1e-10 hold the digits that the
-    small coefficient holds (a hundred roundings of the large one)."""
-    rs = np.random.RandomState(D)
-    U, V = (np.linalg.qr(rs.standard_normal((D, D)) + 1j * rs.standard_normal((D, D)))[0] for _ in range(2))
-    M = np.linalg.qr(rs.standard_normal((D, D)) + 1j * rs.standard_normal((D, D)))[0]
-    s = np.zeros(D)
-    s[:2] = np.cos(small), np.sin(small)
-    psi = ctx.mps([np.asfortranarray((U * s @ M).reshape(D, 1, D)), np.asfortranarray((M.conj().T @ V).T.reshape(D, D, 1))])
-    got = ctx.entropy(psi, 1)
-    psi.free()
-    t = np.sin(small) ** 2
-    want = -(1 - t) * np.log1p(-t) / np.log(2) - (t * np.log2(t) if t > 1e-12 else 0.0)
-    assert abs(got / want - 1.0) < 2 * 100 * 2.2e-16 / small
