@@ -402,10 +402,12 @@ mpsgpu_status mpsgpu_server_submit(mpsgpu_server* srv, const mpsgpu_request* req
 /* Moves up to cap finished results into out (in completion order). */
 mpsgpu_status mpsgpu_server_poll(mpsgpu_server* srv, mpsgpu_result* out, int cap, int* n);
 /* Cancels a queued request, or stops a running one between two site steps.  A
- * request that finished before the call, but whose result has not been polled
- * yet, is reported as cancelled too (its other result fields stand), so that
- * the outcome of a cancel does not depend on how fast the solve was.
- * MPSGPU_INVALID: an id that is unknown or already polled. */
+ * request that finished with success before the call, but whose result has not
+ * been polled yet, is reported as cancelled too (its other result fields, the
+ * energy among them, stand), so that the outcome of a cancel does not depend on
+ * how fast the solve was.  MPSGPU_INVALID: an id that is unknown, already
+ * polled, already cancelled, or whose request ended with an error (its status
+ * stands). */
 mpsgpu_status mpsgpu_server_cancel(mpsgpu_server* srv, uint64_t id);
 /* Waits until no request is queued or running (timeout_s <= 0: no limit). */
 mpsgpu_status mpsgpu_server_drain(mpsgpu_server* srv, double timeout_s);

@@ -331,8 +331,9 @@ mpsgpu_status mpsgpu_server_cancel(mpsgpu_server* s, uint64_t id) {
     raise_cancel(*a->second);
     return MPSGPU_OK;
   }
-  for (auto& res : s->done) {  // finished, its result not collected yet
-    if (res.id == id) {
+  // finished, its result not collected yet; an error, or an earlier cancel, stands
+  for (auto& res : s->done) {
+    if (res.id == id && res.status == MPSGPU_OK) {
       res.status = MPSGPU_CANCELLED;
       return MPSGPU_OK;
     }

@@ -137,3 +137,19 @@ def test_time_evolution_request_alone_and_in_the_mix(tmp_path):
         H = c.mpo_ising(L, 1.0, g, 0.1)
         e = c.contract(saved, H, saved).real / c.contract(saved, None, saved).real
         assert abs(e - alone["energy"]) <= 1e-10 * abs(e)
+
+
+def test_cancel_leaves_errors_and_earlier_cancels(tmp_path):
+    """A request that ended with an error keeps its status, and neither it nor a cancelled one can be cancelled again."""
+    from mpsdyn_b200 import capi
+    CANCELLED = 6
+    with capi.Server(0, slots=1) as srv:
+        failed = srv.submit(ISING, 8, 8, 1.0, 1.0, 0.0, 4, result_file=tmp_path / "missing" / "x.mps")
+        queued = srv.submit(ISING, 8, 8, 1.0, 1.0, 0.0, 5)
+        srv.cancel(queued)
+        srv.drain()
+        for rid in (failed, queued):
+            with pytest.raises(capi.MpsgpuError):
+                srv.cancel(rid)
+        res = {r["id"]: r["status"] for r in _wait(srv, 2)}
+    assert res[failed] not in (0, CANCELLED) and res[queued] == CANCELLED
