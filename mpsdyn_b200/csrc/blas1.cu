@@ -98,8 +98,8 @@ __global__ void wcontract_wide_kernel(WContractArgs a) {
 constexpr int DOT_CHUNK = 4096;
 
 // partial[j * nblk + b] = sum over rows of chunk b of conj(V[:, j]) w
-__global__ void cgemv_c_partial(int n, int k, const cplx* __restrict__ V, long long ldv,
-                                const cplx* __restrict__ w, cplx* __restrict__ partial, int nblk) {
+__global__ void cgemv_c_partial(int n, int k, const cplx* V, long long ldv,
+                                const cplx* w, cplx* __restrict__ partial, int nblk) {
   join_stream();
   __shared__ double rs[TPB / 32], is[TPB / 32];
   const int b = blockIdx.x, j = blockIdx.y;
@@ -121,7 +121,7 @@ __global__ void cgemv_c_partial(int n, int k, const cplx* __restrict__ V, long l
   }
 }
 
-__global__ void reduce_partials(int k, int nblk, const cplx* __restrict__ partial, cplx* __restrict__ out) {
+__global__ void reduce_partials(int k, int nblk, const cplx* partial, cplx* __restrict__ out) {
   join_stream();
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= k) return;
@@ -130,8 +130,8 @@ __global__ void reduce_partials(int k, int nblk, const cplx* __restrict__ partia
   out[j] = s;
 }
 
-__global__ void cgemv_n_sub_kernel(int n, int k, const cplx* __restrict__ V, long long ldv,
-                                   const cplx* __restrict__ h, cplx* __restrict__ w, double sign) {
+__global__ void cgemv_n_sub_kernel(int n, int k, const cplx* V, long long ldv,
+                                   const cplx* h, cplx* __restrict__ w, double sign) {
   join_stream();
   __shared__ cplx hs[256];
   for (int t = threadIdx.x; t < k; t += blockDim.x) hs[t] = h[t];
@@ -144,7 +144,7 @@ __global__ void cgemv_n_sub_kernel(int n, int k, const cplx* __restrict__ V, lon
   }
 }
 
-__global__ void nrm2_partial(int n, const cplx* __restrict__ x, double* __restrict__ partial) {
+__global__ void nrm2_partial(int n, const cplx* x, double* __restrict__ partial) {
   join_stream();
   __shared__ double rs[TPB / 32];
   const int r0 = blockIdx.x * DOT_CHUNK, r1 = min(n, r0 + DOT_CHUNK);
@@ -161,7 +161,7 @@ __global__ void nrm2_partial(int n, const cplx* __restrict__ x, double* __restri
   }
 }
 
-__global__ void nrm2_final(int nblk, const double* __restrict__ partial, double* __restrict__ out) {
+__global__ void nrm2_final(int nblk, const double* partial, double* __restrict__ out) {
   join_stream();
   if (threadIdx.x == 0 && blockIdx.x == 0) {
     double s = 0.0;
@@ -170,7 +170,7 @@ __global__ void nrm2_final(int nblk, const double* __restrict__ partial, double*
   }
 }
 
-__global__ void zscal_inv_kernel(int n, const cplx* __restrict__ x, const double* __restrict__ nrm,
+__global__ void zscal_inv_kernel(int n, const cplx* x, const double* nrm,
                                  cplx* __restrict__ y) {
   join_stream();
   const double inv = 1.0 / nrm[0];
@@ -179,14 +179,14 @@ __global__ void zscal_inv_kernel(int n, const cplx* __restrict__ x, const double
     y[i] = cscale(x[i], inv);
 }
 
-__global__ void zaxpby_kernel(int n, cplx a, const cplx* __restrict__ x, cplx b, cplx* __restrict__ y) {
+__global__ void zaxpby_kernel(int n, cplx a, const cplx* x, cplx b, cplx* __restrict__ y) {
   join_stream();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x)
     y[i] = cadd(cmul(a, x[i]), cmul(b, y[i]));
 }
 
-__global__ void zcopy_kernel(long long n, const cplx* __restrict__ s, cplx* __restrict__ d) {
+__global__ void zcopy_kernel(long long n, const cplx* s, cplx* __restrict__ d) {
   join_stream();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x)
@@ -228,7 +228,7 @@ __global__ void site_dev_to_ref_kernel(int d, int Dl, int Dr, const cplx* __rest
   }
 }
 
-__global__ void transpose_pqr_kernel(int P, int Q, int R, const cplx* __restrict__ in,
+__global__ void transpose_pqr_kernel(int P, int Q, int R, const cplx* in,
                                      cplx* __restrict__ out, bool conj) {
   join_stream();
   const long long n = (long long)P * Q * R;
@@ -278,7 +278,7 @@ __device__ __forceinline__ long long view_off(const View2& v, long long i, long 
   return (i % v.rd) * v.r0 + (i / v.rd) * v.r1 + (j % v.cd) * v.c0 + (j / v.cd) * v.c1;
 }
 
-__global__ void gather2_kernel(int m, int n, const cplx* __restrict__ src, View2 v,
+__global__ void gather2_kernel(int m, int n, const cplx* src, View2 v,
                                cplx* __restrict__ dst) {
   join_stream();
   const long long tot = (long long)m * n;
@@ -291,7 +291,7 @@ __global__ void gather2_kernel(int m, int n, const cplx* __restrict__ src, View2
   }
 }
 
-__global__ void scatter2_kernel(int m, int n, const cplx* __restrict__ src, cplx* __restrict__ dst,
+__global__ void scatter2_kernel(int m, int n, const cplx* src, cplx* __restrict__ dst,
                                 View2 v) {
   join_stream();
   const long long tot = (long long)m * n;

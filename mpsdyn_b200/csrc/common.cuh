@@ -147,6 +147,9 @@ inline void after_launch(const Stream& st) {
 // await_predecessor() before it touches memory, in every thread: that waits for
 // the predecessor's end and its writes, so only the launch itself overlaps (a
 // ground state at L = 48, D = 64 174 -> 158 ms, a quench at D = 16 48 -> 37 ms).
+// Its inputs are plain pointers, not const __restrict__, and it uses no __ldg: both
+// say that no one writes the data while the kernel lives, which the predecessor
+// may do until it ends.
 // A predecessor that calls admit_successor() lets the next kernel's blocks become
 // resident from there on, beside its own.  Both only for grids of up to half the
 // SMs, which find SMs of their own: admitted early, the blocks of a larger grid

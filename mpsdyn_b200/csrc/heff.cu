@@ -365,7 +365,7 @@ __global__ void __launch_bounds__(nthreads<BM>(), BM <= 32 ? 3 : 2) heff_gemm1w_
     for (int o = tid; o < nout; o += NT_) ooff[o] = (o % d.n_o0) * d.so0 + (o / d.n_o0) * d.so1;
     for (int i = tid; i < kp; i += NT_) ioff[i] = i < nin ? TX * (i % d.n_i0) * LD + i / d.n_i0 : -1;
     __syncthreads();
-    for (int e = tid; e < nw; e += NT_) Ws[leg_index(e, wld)] = __ldg(&d.Wm[e]);
+    for (int e = tid; e < nw; e += NT_) Ws[leg_index(e, wld)] = __ldcg(&d.Wm[e]);
     acc_to_smem<BM, BN, NS>(acc, Cs);  // ends with a barrier
     const int lane = tid & 31, fr = lane >> 2, fc = lane & 3;
     for (int u = tid >> 5; u < np8 * no8; u += NT_ / 32) {
@@ -394,7 +394,7 @@ __global__ void __launch_bounds__(nthreads<BM>(), BM <= 32 ? 3 : 2) heff_gemm1w_
   const cplx* Wp = d.Wm;
   if (nw * (int)sizeof(cplx) <= ROOM) {
     cplx* Ws = Cs + BM * LD;
-    for (int e = tid; e < nw; e += NT_) Ws[leg_index(e, nout)] = __ldg(&d.Wm[e]);
+    for (int e = tid; e < nw; e += NT_) Ws[leg_index(e, nout)] = __ldcg(&d.Wm[e]);
     Wp = Ws;
   }
   acc_to_smem<BM, BN, NS>(acc, Cs);

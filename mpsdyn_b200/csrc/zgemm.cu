@@ -36,7 +36,7 @@ constexpr int BK = 16;
 constexpr int PAD = 4;
 
 template <int OP>
-__device__ __forceinline__ cplx load_op(const cplx* __restrict__ p, long long idx) {
+__device__ __forceinline__ cplx load_op(const cplx* p, long long idx) {
   cplx v = p[idx];
   if (OP == OP_C) v.y = -v.y;
   return v;
@@ -58,7 +58,7 @@ struct TileSmem {
 // the caller's accumulators acc[i][j][set][h] (set: 0 re*re, 1 -im*im,
 // 2 re*im, 3 im*re).
 template <int BM, int BN, int WMW, int WNW, int OPA, int OPB>
-__device__ __forceinline__ void gemm_tile(const cplx* __restrict__ A, long long lda, const cplx* __restrict__ B,
+__device__ __forceinline__ void gemm_tile(const cplx* A, long long lda, const cplx* B,
                                           long long ldb, int M, int N, int m0, int n0, int kbeg, int kend,
                                           TileSmem<BM, BN>& sm,
                                           double (&acc)[BM / WMW / 8][BN / WNW / 8][4][2]) {
@@ -217,7 +217,7 @@ zgemm_dmma_kernel(GemmArgs g, int splits, int kchunk, cplx* __restrict__ partial
   }
 }
 
-__global__ void splitk_reduce_kernel(GemmArgs g, int splits, const cplx* __restrict__ partial) {
+__global__ void splitk_reduce_kernel(GemmArgs g, int splits, const cplx* partial) {
   join_stream();
   long long mn = (long long)g.M * g.N;
   long long total = mn * g.batch;
