@@ -128,20 +128,20 @@ __device__ __forceinline__ bool jacobi_pair(cplx* ap, cplx* aq, int m, cplx* vp,
       return true;
     }
   }
-  const double g2 = cabs2(ga), ab = al * be;
-  double g = sqrt(g2);
+  const double ab = al * be;
+  double g2 = cabs2(ga), sc = 1.0;
   if (g2 < 2.3e-308) {
-    // |gamma| from its larger part: the root of a square below the normal range,
-    // and with it the modulus of the phase below, is off by up to 40 %, and the
-    // column it multiplies may be a large one (a second value of 1.7e-6 beside
+    // below the normal range from the product times 2^200: the root of the square
+    // itself, and with it the modulus of the phase below, is off by up to 40 %, and
+    // the column it multiplies may be a large one (a second value of 1.7e-6 beside
     // columns of 1e-150 came out 20 % off).  Where the square vanishes the pair is
-    // left alone: settling values below 1e-81 can
-    // take more than the 40 sweeps (44 at 300 columns graded over ten decades).
-    const double mx = fmax(fabs(ga.x), fabs(ga.y));
-    if (!(mx >= 2.3e-162)) return false;
-    const double x = ga.x / mx, y = ga.y / mx;
-    g = mx * sqrt(fma(x, x, y * y));
+    // left alone: settling values below 1e-81 can take more than the 40 sweeps (44
+    // at 300 columns graded over ten decades).
+    if (!(g2 > 0.0)) return false;
+    g2 = cabs2(cscale(ga, 0x1p200));
+    sc = 0x1p-200;
   }
+  const double g = sqrt(g2) * sc;
   // (ab underflows for two columns of 1e-80, each square does not)
   if (!(g > JTOL * (ab > 1e-280 ? sqrt(ab) : sqrt(al) * sqrt(be)))) return false;
   // rotate (a_p, a_q conj(phase)) so that the pair becomes orthogonal
