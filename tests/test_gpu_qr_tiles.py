@@ -37,3 +37,12 @@ def test_qr_degenerate_columns(ctx, m, n, zero):
     for j in range(n):  # each column at its own scale
         scale = max(np.abs(A[:, j]).max(), 1e-300)
         assert np.abs((Q @ (R[:, j] / scale)) - A[:, j] / scale).max() < 1e-12
+
+
+@pytest.mark.parametrize("m,n", [(32, 8), (40, 8), (70, 1), (300, 5)])
+def test_qr_of_nan_is_nan(ctx, m, n):
+    """A column of NaN below a finite pivot is no column of zeros for the cluster forms: R shows it."""
+    A = np.random.default_rng(m).standard_normal((m, n)) + 0j
+    A[1:, 0] = complex(np.nan, np.nan)
+    Q, R = ctx.qr(A)
+    assert np.isnan(R[0, 0]) and np.isnan(Q[:, 0]).any()
