@@ -530,11 +530,11 @@ void lanczos_combine(const Stream& st, LzCombineBatch& b, cplx* ws, unsigned* ba
   }
   b.pn = reinterpret_cast<double*>(ws);
   b.bar = bars + parity * LZ_MAXI * PHASES;
-  parity ^= 1;
-  b.bar_next = bars + parity * LZ_MAXI * PHASES;
+  b.bar_next = bars + (parity ^ 1) * LZ_MAXI * PHASES;
   void* args[] = {&b};
   MPSGPU_CUDA(cudaLaunchCooperativeKernel((void*)lanczos_combine_kernel, dim3(c0), dim3(T), args, 0, st.s));
   after_launch(st);
+  parity ^= 1;  // a launch that failed has not cleared the other set
 }
 
 void lanczos_step(const Stream& st, LzBatch& b, cplx* ws, unsigned* bars, int& parity) {
@@ -597,8 +597,7 @@ void lanczos_step(const Stream& st, LzBatch& b, cplx* ws, unsigned* bars, int& p
   b.pn1 = reinterpret_cast<double*>(b.part2 + (long long)G * KMAXS);
   b.pn2 = b.pn1 + G;
   b.bar = bars + parity * LZ_MAXI * PHASES;
-  parity ^= 1;
-  b.bar_next = bars + parity * LZ_MAXI * PHASES;
+  b.bar_next = bars + (parity ^ 1) * LZ_MAXI * PHASES;
   // algorithmic bytes: the basis read twice (projections, update), w read
   // and written three times (three-term step, update, normalisation) and
   // v_{j-1} once; the projector vectors twice
@@ -610,6 +609,7 @@ void lanczos_step(const Stream& st, LzBatch& b, cplx* ws, unsigned* bars, int& p
   MPSGPU_CUDA(cudaLaunchCooperativeKernel(res ? (void*)lanczos_step_kernel<true> : (void*)lanczos_step_kernel<false>,
                                           dim3(c0), dim3(T), args, 0, st.s));
   after_launch(st);
+  parity ^= 1;  // a launch that failed has not cleared the other set
 }
 
 }  // namespace mpsgpu
