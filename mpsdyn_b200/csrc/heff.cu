@@ -63,6 +63,12 @@ template <int BM>
 __host__ __device__ constexpr int kgroups() { return BM <= 32 ? 2 : 1; }
 template <int BM>
 __host__ __device__ constexpr int nthreads() { return 128 * kgroups<BM>(); }
+// CTAs per SM that the registers are cut for.  Two for four accumulators: cut for
+// three they spilled 150 bytes in launches of few blocks, which are bound by latency
+// (both products of a site at D = 16, w = 3, one or sixteen problems: 12.3 -> 10.3 us and
+// 14.3 -> 12.3 us; of 192 problems 22.5 -> 23.0 us).
+template <int BM, int NS>
+__host__ __device__ constexpr int ctas_per_sm() { return BM > 32 || NS == 4 ? 2 : 3; }
 
 __device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b) {
   asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
@@ -311,7 +317,7 @@ struct Source<Extern<D>> {
 // heff_gemm1w
 // ---------------------------------------------------------------------------
 template <int BM, int BN, int NS, class B>
-__global__ void __launch_bounds__(nthreads<BM>(), BM <= 32 ? 3 : 2) heff_gemm1w_kernel(const __grid_constant__ B b) {
+__global__ void __launch_bounds__(nthreads<BM>(), ctas_per_sm<BM, NS>()) heff_gemm1w_kernel(const __grid_constant__ B b) {
   __shared__ typename Source<B>::Slot slot;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int NT_ = nthreads<BM>();
@@ -429,7 +435,7 @@ __global__ void __launch_bounds__(nthreads<BM>(), BM <= 32 ? 3 : 2) heff_gemm1w_
 // heff_gemm3 (cluster split-K)
 // ---------------------------------------------------------------------------
 template <int BM, int BN, int CS, int NS, class B>
-__global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(nthreads<BM>(), BM <= 32 ? 3 : 2)
+__global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(nthreads<BM>(), ctas_per_sm<BM, NS>())
     heff_gemm3_kernel(const __grid_constant__ B b) {
   __shared__ typename Source<B>::Slot slot;
   extern __shared__ __align__(16) unsigned char smem_raw[];
