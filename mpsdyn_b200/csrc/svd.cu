@@ -167,8 +167,8 @@ __device__ __forceinline__ int circle_item(int k, int step, int n) {
 // A: m x n (n even; n a multiple of 16 with more than one CTA), column-major,
 // ld m, rotated in place.  V (n x n, ld n, identity on entry) accumulates the
 // rotations when non-null, so that A_in V = A_out.  out: n column norms;
-// status[0] = sweeps used (MAX_SWEEPS + 1 if not converged), status[1 + s]
-// zero on entry (rotations left in sweep s).  gridDim.x = n / 16 CTAs (at least 1).
+// status[0] = sweeps used (MAX_SWEEPS + 1 if not converged), with more than one
+// CTA status[1 + s] zero on entry (rotations left in sweep s).  gridDim.x = n / 16 CTAs (at least 1).
 // SMALL (one CTA): sums, tests and rotations in the order and form of the
 // unblocked algorithm.
 template <bool SMALL, int SYNC>
@@ -209,6 +209,7 @@ __global__ void __launch_bounds__(JT) jacobi_sv_kernel(int m, int n, cplx* A, cp
   if (SYNC == JSYNC_NONE) columns(0, 0, true);
   const int rounds = SYNC == JSYNC_NONE ? 1 : nblk - 1;
   int sweep = 0;
+  bool any = false;
   for (; sweep < MAX_SWEEPS; sweep++) {
     for (int rd = 0; rd < rounds; rd++) {
       int b0 = 0, b1 = 0;
@@ -232,13 +233,14 @@ __global__ void __launch_bounds__(JT) jacobi_sv_kernel(int m, int n, cplx* A, cp
           __syncthreads();
         }
       }
-      if (rotated) {  // written before the last barrier
-        if (SYNC != JSYNC_NONE) columns(b0, b1, false);
+      any = rotated;  // written before the last barrier
+      if (SYNC != JSYNC_NONE && any) {
+        columns(b0, b1, false);
         if (tid == 0) atomicOr(&status[1 + sweep], 1);
       }
       everyone();
     }
-    if (__ldcg(&status[1 + sweep]) == 0) break;
+    if (SYNC == JSYNC_NONE ? !any : __ldcg(&status[1 + sweep]) == 0) break;
   }
   if (SYNC == JSYNC_NONE) {
     columns(0, 0, false);
@@ -361,8 +363,10 @@ void jacobi_launch(const Stream& st, int rows, int colsp, cplx* W, cplx* V, doub
     g_jac_cluster[dev].store(best);
     mark_device_done(g_jac_setup);
   }
-  MPSGPU_CUDA(cudaMemsetAsync(d_status, 0, JSTATUS, st.s));
-  if (smem > JSMEM) {
+  const bool longc = smem > JSMEM, one_cta = longc || colsp <= 2 * NBJ;
+  // (one CTA keeps its flag in shared memory)
+  if (!one_cta) MPSGPU_CUDA(cudaMemsetAsync(d_status, 0, JSTATUS, st.s));
+  if (longc) {
     jacobi_long_kernel<<<1, JLT, 0, st.s>>>(rows, colsp, W, V, d_sig, d_status);
   } else if (colsp <= 2 * NBJ) {
     small<<<1, JT, smem, st.s>>>(rows, colsp, W, V, d_sig, d_status);
