@@ -3000,7 +3000,7 @@ static bool schmidt_two_chains(Context& c, const MpsDev& s, int pos, std::vector
     int kl = 0, kr = 0;
     const int D = s.dims[pos][1];
     double nrm[2];
-    std::vector<cplx> diag[2];  // of the factors
+    std::vector<cplx> diag[2];  // of the factors, where the side is a choice (20 us)
     {
       SecondStream two(c);
       Context& o = two.sub;
@@ -3022,10 +3022,9 @@ static bool schmidt_two_chains(Context& c, const MpsDev& s, int pos, std::vector
       two.join();
       MPSGPU_CUDA(cudaMemcpyAsync(&nrm[0], c.dscal, sizeof(double), cudaMemcpyDeviceToHost, c.stream));
       MPSGPU_CUDA(cudaMemcpyAsync(&nrm[1], o.dscal, sizeof(double), cudaMemcpyDeviceToHost, c.stream));
-      for (int i = 0; i < 2; i++) {
-        const int k = i ? kr : kl;
-        diag[i].resize(std::min(k, D));
-        MPSGPU_CUDA(cudaMemcpy2DAsync(diag[i].data(), sizeof(cplx), i ? o.matR.p : c.matR.p, (k + 1) * sizeof(cplx),
+      for (int i = 0; i < 2 && kl == kr && kl > 16; i++) {
+        diag[i].resize(std::min(kl, D));
+        MPSGPU_CUDA(cudaMemcpy2DAsync(diag[i].data(), sizeof(cplx), i ? o.matR.p : c.matR.p, (kl + 1) * sizeof(cplx),
                                       sizeof(cplx), diag[i].size(), cudaMemcpyDeviceToHost, c.stream));
       }
       MPSGPU_CUDA(cudaStreamSynchronize(c.stream));
