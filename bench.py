@@ -171,7 +171,10 @@ def run_reference(args, rank: int, world: int) -> None:
     procs = min(os.cpu_count() or 1, 64)
     vals, walls, last = [], [], None
     for _ in range(max(1, args.steps)):  # no warm-up: nothing on the CPU path warms up
-        v, sample, detail = reference_rate(procs, args.ref_iter_cap)
+        try:
+            v, sample, detail = reference_rate(procs, args.ref_iter_cap)
+        except FileNotFoundError as e:  # the reference was not built here (no sources)
+            v, sample = None, str(e)
         if v is None:
             print(json.dumps({"impl": "reference", "unavailable": sample}), flush=True)
             return
