@@ -235,7 +235,7 @@ __device__ __noinline__ void qc_panel(const QcParams& p, const cplx* As, int pn,
 #pragma unroll
       for (int i = 0; i < RPL; i++) mx = fmax(mx, fmax(fabs(x[i].x), fabs(x[i].y)));
       for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-      identity = mx == 0.0 && n2 == 0.0 && alpha.y == 0.0;  // (the maximum passes NaN by, n2 does not)
+      identity = mx == 0.0 && alpha.y == 0.0 && nrm2 == nrm2;  // (the maximum passes NaN by)
       if (identity) break;
       // divided by a power of two near the largest component (at least the smallest normal)
       const int top = __double2hiint(fmax(mx, fmax(fabs(alpha.x), fabs(alpha.y)))) & 0x7ff00000;
