@@ -224,10 +224,10 @@ def bf16_peak() -> tuple:
 
 
 # dram__bytes_read.sum + dram__bytes_write.sum per launch from ncu captures of
-# the same shapes (profiles/), None where none was taken: the Lanczos step of
-# eight D = 128 Schwinger chains (one launch of the lockstep sample),
-# profiles/lanczos_step_heff_schwinger_sample_N40_D128_batch8.md
-KERNEL_TRAFFIC = {"gemm_fp64_dmma": None, "gemm_split_tcgen05": None, "lanczos_step": 102.5e6, "qr": 0.667e6,
+# the same shapes, None where none was taken: the Lanczos step of eight D = 128
+# Schwinger chains and the QR of a 256 x 128 site (one launch of the lockstep
+# sample each), profiles/kernels_schwinger_sample_N40_D128_batch8.md
+KERNEL_TRAFFIC = {"gemm_fp64_dmma": None, "gemm_split_tcgen05": None, "lanczos_step": 84.3e6, "qr": 0.613e6,
                   "split_operands": None}
 
 

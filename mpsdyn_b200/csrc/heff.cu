@@ -34,8 +34,8 @@
 //     slab instead of recomputing rows, columns and edges for every copy
 //     (gemm3, eight problems at D = 96: 31.3 us -> 28.9 us);
 //   - the leg epilogue is itself a product, pixels x legs, on the DMMA from
-//     shared memory with offsets in tables; as scalar code it took 25 us of the
-//     84 us of eight problems at D = 128, w = 5, now 8 us of 67 us.
+//     shared memory with offsets in tables (with it as scalar code eight problems
+//     at D = 128, w = 5 took 84 us, now 67 us).
 // Measured now: D = 128, w = 5, eight problems 67 and 57 us (20 and 23.5 TF), one
 // 20.6 and 14.5 us; D = 64, w = 3, one 10.3 and 8.3 us; D = 400, w = 3, four 446
 // and 440 us (28 TF).

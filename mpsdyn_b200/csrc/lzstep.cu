@@ -23,7 +23,11 @@
 // writes one partial sum per vector.  After one barrier among the instance's
 // CTAs each of them adds the partials of the instance in the same fixed order,
 // so all hold the same coefficients and reach the same second-pass decision.
-// An unflagged step costs that one barrier.
+// An unflagged step costs that one barrier.  How many rows a CTA takes, and
+// whether the basis goes to registers, follows the whole group of a launch: the
+// order of an instance's sums, and so its rounding, depends on the instances beside
+// it (as the contractions' split of K does), and a chain agrees with the same chain
+// alone to the solver's tolerance, not to the last bit.
 //
 // Small groups (at most 64 rows per CTA with one CTA per SM slot, and k <= 64)
 // are bound by latency, not by bytes: a launch, the chain w -> dots -> barrier

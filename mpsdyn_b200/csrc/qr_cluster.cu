@@ -25,11 +25,9 @@
 // in 80 us, 64 x 32 in 37 us, 256 x 256 in 415 us, 512 x 256 in 776 us.  Slices of
 // 16 columns, two to a warp and two barriers a column, took 284, 111, 47, 620 and
 // 767 us, a row per thread with sums folded over the lanes 317 us at 256 x 128, the
-// global-memory kernels of qr.cu 3560 us at 512 x 256.  A column of a 256-row panel
-// takes 2000 cycles: 500 the update of the next pivot column and its way to shared
-// memory, 900 reading it back, the products and the shuffles, 450 square root,
-// reciprocals and factors.  A block application takes 5300 (2050 on the FP64 tensor
-// pipe), Q 4500 a panel.
+// global-memory kernels of qr.cu 3560 us at 512 x 256.  At 256 x 128 a warp waits
+// 29 cycles at barriers for every instruction that it issues, and the FP64 tensor pipe
+// is active 7 % of the time.
 #include <cooperative_groups.h>
 
 #include "common.cuh"

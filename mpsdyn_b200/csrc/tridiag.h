@@ -206,8 +206,9 @@ inline double tridiag_eigenvalue(const std::vector<double>& a, const std::vector
 }
 
 // All eigenvalues of the k x k tridiagonal (a, b), ascending, by implicit-shift
-// QL (Dubrulle, Martin & Wilkinson, Numer. Math. 12, 1968): O(k^2), where a
-// bisection per value takes forty chains of k divisions each.  False when an
+// QL (Dubrulle, Martin & Wilkinson, Numer. Math. 12, 1968; in the form of EISPACK's
+// imtql1, which is in the public domain): O(k^2), where a bisection per value takes
+// forty chains of k divisions each.  False when an
 // off-diagonal element does not vanish within 60 sweeps.
 inline bool tridiag_all_values(const std::vector<double>& a, const std::vector<double>& b, int k, double scale,
                                std::vector<double>& d, std::vector<double>& e) {
