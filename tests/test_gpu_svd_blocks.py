@@ -137,3 +137,29 @@ def test_values_of_tiny_matrices(ctx, D, scale):
     phi.free()
     s = np.linalg.svd(G, compute_uv=False)
     assert abs(discarded / scale / scale / np.sum(s[cut:] ** 2) - 1.0) < 1e-12
+
+
+@pytest.mark.parametrize("order", ["mixed", "rising"])
+@pytest.mark.parametrize("L,D,low", [(12, 64, 60), (14, 128, 100), (16, 256, 60)])
+def test_unsorted_gradings_settle(ctx, L, D, low, order):
+    """A bond whose coefficients fall over many orders in no order, or rise: Schmidt values and a cut settle."""
+    rs = np.random.RandomState(5)
+    s = 10.0 ** -np.linspace(0, low, D)
+    s = s[rs.permutation(D)] if order == "mixed" else s[::-1]
+    bond = [min(D, 2 ** min(k, L - k)) for k in range(L + 1)]
+    sites = []
+    for k, (a, r) in enumerate(zip(bond, bond[1:])):
+        if k < L // 2:
+            A = np.linalg.qr(rs.standard_normal((2 * a, r)) + 1j * rs.standard_normal((2 * a, r)))[0].reshape(2, a, r)
+        else:
+            A = np.linalg.qr(rs.standard_normal((2 * r, a)) + 1j * rs.standard_normal((2 * r, a)))[0]
+            A = A.conj().T.reshape(a, 2, r).transpose(1, 0, 2)
+        sites.append(np.asfortranarray(s[None, :, None] * A if k == L // 2 else A))
+    psi = ctx.mps(sites)
+    want = np.sort(s**2 / np.sum(s**2))[::-1]
+    phi, discarded = psi.approximate(D // 2)
+    for state in (psi, phi):
+        got = np.sort(ctx.schmidt_values(state, L // 2))[::-1][: D // 2]
+        assert np.max(np.abs(got - want[: D // 2])) < 1e-12
+        state.free()
+    assert 0.0 <= discarded < 1e-24
