@@ -131,7 +131,8 @@ __device__ __forceinline__ bool jacobi_pair(cplx* ap, cplx* aq, int m, cplx* vp,
     }
   }
   const double ab = al * be;
-  double g2 = cabs2(ga), sc = 1.0;
+  const double g2 = cabs2(ga);
+  double g = sqrt(g2);
   if (g2 < 2.3e-308) {
     // below the normal range from the product times 2^200: the root of the square
     // itself, and with it the modulus of the phase below, is off by up to 40 %, and
@@ -140,10 +141,8 @@ __device__ __forceinline__ bool jacobi_pair(cplx* ap, cplx* aq, int m, cplx* vp,
     // left alone: values below 1e-81, which no one asks for beside larger ones, would
     // take up to 30 sweeps more.
     if (!(g2 > 0.0)) return false;
-    g2 = cabs2(cscale(ga, 0x1p200));
-    sc = 0x1p-200;
+    g = sqrt(cabs2(cscale(ga, 0x1p200))) * 0x1p-200;
   }
-  const double g = sqrt(g2) * sc;
   // (ab underflows for two columns of 1e-80, each square does not)
   if (!(g > JTOL * (ab > 1e-280 ? sqrt(ab) : sqrt(al) * sqrt(be)))) return false;
   // rotate (a_p, a_q conj(phase)) so that the pair becomes orthogonal
